@@ -211,20 +211,23 @@ void fill_tables(SpecTables<T> &S, const cc_params *p) {
     const double mw = p->mw[k];
     S.mw[k] = (T)mw;
     S.inv_mw[k] = (T)(1.0 / mw);
-    S.r_over_mw[k] = (T)(kRu / mw);
     S.cv_shift[k] = (T)(kRu / mw);
     S.t_low[k] = (T)p->t_low[k];
     S.t_mid[k] = (T)p->t_mid[k];
     const double *lo = p->low_temp_coeff + 7 * k, *hi = p->high_temp_coeff + 7 * k;
-    const double sc[5] = {1.0, 0.5, 1.0 / 3.0, 0.25, 0.2};
-    for (int r = 0; r < 2; ++r) {
-      const double *a = r == 0 ? lo : hi;
-      T *rec = S.rec[k][r];
-      for (int c = 0; c < 5; ++c) rec[c] = (T)a[c], rec[5 + c] = (T)(a[c] * sc[c]);
-      rec[7] = (T)(a[2] / 3);
-      rec[10] = (T)a[5];
-      rec[11] = 0;
-    }
+    const double r = kRu / mw, tl = p->t_low[k];
+    for (int q = 0; q < 6; ++q) S.rec[k][1][q] = (T)(r * lo[q]), S.rec[k][2][q] = (T)(r * hi[q]);
+    // below t_low: cp(t_low), and h continued linearly from h(t_low)
+    const double cp = lo[0] + tl * (lo[1] + tl * (lo[2] + tl * (lo[3] + tl * lo[4])));
+    const double h =
+        lo[5] + tl * (lo[0] + tl * (lo[1] / 2 + tl * (lo[2] / 3 + tl * (lo[3] / 4 + tl * (lo[4] / 5)))));
+    S.rec[k][0][0] = (T)(r * cp);
+    S.rec[k][0][5] = (T)(r * (h - cp * tl));
+    const T high = std::max(S.t_low[k], S.t_mid[k]);
+    S.t_low_min = k == 0 ? S.t_low[k] : std::min(S.t_low_min, S.t_low[k]);
+    S.t_low_max = k == 0 ? S.t_low[k] : std::max(S.t_low_max, S.t_low[k]);
+    S.t_mid_min = k == 0 ? S.t_mid[k] : std::min(S.t_mid_min, S.t_mid[k]);
+    S.t_high_max = k == 0 ? high : std::max(S.t_high_max, high);
     S.lj_inv[k] = (T)p->LJ_potent_inv[k];
     S.vis_coeff[k] = (T)p->vis_coeff[k];
     S.lam_shift[k] = (T)(1.25 * kRu / mw);

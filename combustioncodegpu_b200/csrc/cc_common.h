@@ -11,23 +11,24 @@ constexpr double kMwAir = 28.9647;     // Constants.h:28
 constexpr int kMaxSpec = 16;           // species supported by one context
 constexpr int kTX = 32;                // stage tile: points along i (one warp)
 constexpr int kTY = 8;                 // stage tile: points along j (warps)
-constexpr int kRecLen = 12;            // values per NASA-7 record (cp, h, pad)
+constexpr int kRecRanges = 3;          // NASA-7 records per species: T < t_low, t_low <= T < t_mid, T >= t_mid
+constexpr int kRecLen = 8;             // values per NASA-7 record (a0..a5, pad)
 constexpr long long kDefaultWaitSpins = 1LL << 22;  // polls of a device wait before it gives up
 
 // Per-precision species tables, passed to every kernel by value (constant
-// bank).  Horner-form NASA-7 coefficients: for T >= t_mid the `hi` set.
+// bank).
 template <typename T>
 struct SpecTables {
   T mw[kMaxSpec];
   T inv_mw[kMaxSpec];
-  T r_over_mw[kMaxSpec];      // R_u / W_k
-  T cv_shift[kMaxSpec];       // R_u / W_k (cp - cv per species)
+  T cv_shift[kMaxSpec];       // R_u / W_k (gas constant of the species, cp - cv)
   T t_low[kMaxSpec], t_mid[kMaxSpec];
-  // NASA-7 record of species k, range r (0: T < t_mid, 1: T >= t_mid):
-  //   [0..4]  cp/R = a0 + a1 T + ... + a4 T^4
-  //   [5..10] h/R  = a5 + T(a0 + T(a1/2 + T(a2/3 + T(a3/4 + T a4/5)))) as b0..b4 = a0, a1/2, .., a4/5; b5 = a5
-  //   [11]    padding (records are 16-byte aligned for vector loads)
-  alignas(16) T rec[kMaxSpec][2][kRecLen];
+  // bounds over the species: below t_low_min every species is in range 0,
+  // in [t_low_max, t_mid_min) in range 1, from t_high_max on in range 2
+  T t_low_min, t_low_max, t_mid_min, t_high_max;
+  // NASA-7 record of species k, range r, times R_u / W_k: a0..a4 of cp, a5 of
+  // h, and padding (records are 16-byte aligned for vector loads)
+  alignas(16) T rec[kMaxSpec][kRecRanges][kRecLen];
   T lj_inv[kMaxSpec];
   T vis_coeff[kMaxSpec];
   T lam_shift[kMaxSpec];      // 1.25 R_u / W_k

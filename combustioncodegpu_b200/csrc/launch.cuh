@@ -25,7 +25,7 @@ size_t Launch<T, NS>::stage_tma_smem() {
 
 template <typename T, int NS>
 size_t Launch<T, NS>::faces_smem() {
-  return sizeof(T) * SpecCount<NS>::kArr * 2 * kRecLen;
+  return sizeof(T) * SpecCount<NS>::kArr * kRecRanges * kRecLen;
 }
 
 template <typename T, int NS>

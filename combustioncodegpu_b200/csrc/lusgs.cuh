@@ -368,10 +368,10 @@ __global__ void __launch_bounds__(kTX *kTY) k_lusgs_update(const StageArgs<T> a,
   const int ns = SpecCount<NS>::n(C);
   const int nv = 5 + ns;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  double *sRecD = reinterpret_cast<double *>(smem_raw);  // [A][2][kRecLen]
+  double *sRecD = reinterpret_cast<double *>(smem_raw);  // [A][kRecRanges][kRecLen]
   T *sRec = reinterpret_cast<T *>(smem_raw + (sizeof(T) == sizeof(double) ? 0 : StageSmem<T, NS>::kRecD));
   const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * kTX + tx;
-  for (int e = tid, nrec = ns * 2 * kRecLen; e < nrec; e += kTX * kTY) {
+  for (int e = tid, nrec = ns * kRecRanges * kRecLen; e < nrec; e += kTX * kTY) {
     sRecD[e] = param_rec<double>(C)[e];
     if (sizeof(T) != sizeof(double)) sRec[e] = param_rec<T>(C)[e];
   }

@@ -45,71 +45,118 @@ __device__ __forceinline__ double frcp(double a) { return 1.0 / a; }
 __device__ __forceinline__ float frcp(float a) { return __fdividef(1.0f, a); }
 __device__ __forceinline__ double fsqrt(double a) { return sqrt(a); }
 __device__ __forceinline__ float fsqrt(float a) { return a * rsqrtf(a); }
+__device__ __forceinline__ double frsqrt(double a) { return rsqrt(a); }
+__device__ __forceinline__ float frsqrt(float a) { return rsqrtf(a); }
 
 // NASA-7 records (SpecTables::rec) are read through a pointer `rec` to the
-// [kMaxSpec][2][kRecLen] array: the stage kernel points it at a copy in
-// shared memory, other kernels at the constant bank (param_rec).  The range
-// is chosen per thread by the record address, so a warp whose points
+// [kMaxSpec][kRecRanges][kRecLen] array: the stage kernels point it at a copy
+// in shared memory, other kernels at the constant bank (param_rec).  The
+// range is chosen per thread by the record address, so a warp whose points
 // straddle t_mid reads two records in one vector load instead of serialising
 // on divergent constant addresses, and the coefficients cannot be hoisted
 // out of the surrounding loops into registers.
+//
+// A record holds a0..a5 of one range, times R_u / W: cp = a0 + a1 T + .. +
+// a4 T^4 and h = a5 + T (a0 + a1 T/2 + .. + a4 T^4/5), per unit mass.  Below
+// t_low, where h continues linearly with cp(t_low) (Thermo.cu:7-63), both are
+// polynomials of the same form, so range 0 is a record too.
 template <typename T>
 __device__ __forceinline__ const T *param_rec(const ChemParams &C) {
   return &tab<T>(C).rec[0][0][0];
 }
 
 template <typename T>
-__device__ __forceinline__ void load_rec(const T *r, T (&x)[kRecLen]);
+__device__ __forceinline__ void load_rec(const T *r, T (&x)[6]);
 template <>
-__device__ __forceinline__ void load_rec<float>(const float *r, float (&x)[kRecLen]) {
-  const float4 *v = reinterpret_cast<const float4 *>(r);
-#pragma unroll
-  for (int q = 0; q < 3; ++q) {
-    const float4 w = v[q];
-    x[4 * q] = w.x, x[4 * q + 1] = w.y, x[4 * q + 2] = w.z, x[4 * q + 3] = w.w;
-  }
+__device__ __forceinline__ void load_rec<float>(const float *r, float (&x)[6]) {
+  const float4 w = *reinterpret_cast<const float4 *>(r);
+  const float2 y = *reinterpret_cast<const float2 *>(r + 4);
+  x[0] = w.x, x[1] = w.y, x[2] = w.z, x[3] = w.w, x[4] = y.x, x[5] = y.y;
 }
 template <>
-__device__ __forceinline__ void load_rec<double>(const double *r, double (&x)[kRecLen]) {
+__device__ __forceinline__ void load_rec<double>(const double *r, double (&x)[6]) {
   const double2 *v = reinterpret_cast<const double2 *>(r);
 #pragma unroll
-  for (int q = 0; q < 6; ++q) {
+  for (int q = 0; q < 3; ++q) {
     const double2 w = v[q];
     x[2 * q] = w.x, x[2 * q + 1] = w.y;
   }
 }
 
-// Enthalpy and cp of species k at temperature t (per unit mass); below
-// t_low, h continues linearly with cp(t_low) (Thermo.cu:7-63).
+// Record of species k at temperature t.
 template <typename T>
-__device__ __forceinline__ void nasa_h_cp(const SpecTables<T> &S, const T *rec, int k, T t, T &h, T &cp) {
-  const T tl = S.t_low[k];
-  const bool below = t < tl;
-  const T te = below ? tl : t;
-  const bool lo = below || t < S.t_mid[k];
-  T x[kRecLen];
-  load_rec<T>(rec + (2 * k + (lo ? 0 : 1)) * kRecLen, x);
-  const T c = x[0] + te * (x[1] + te * (x[2] + te * (x[3] + te * x[4])));
-  T hh = x[10] + te * (x[5] + te * (x[6] + te * (x[7] + te * (x[8] + te * x[9]))));
-  if (below) hh += c * (t - te);
-  h = hh * S.r_over_mw[k];
-  cp = c * S.r_over_mw[k];
+__device__ __forceinline__ const T *species_rec(const SpecTables<T> &S, const T *rec, int k, T t) {
+  const int r = t < S.t_low[k] ? 0 : (t < S.t_mid[k] ? 1 : 2);
+  return rec + (kRecRanges * k + r) * kRecLen;
+}
+
+// The range of every species at temperature t at once, or -1 where they
+// differ: with the usual tables (one t_low and t_mid for all species) two
+// comparisons serve the whole mixture.
+template <typename T>
+__device__ __forceinline__ int common_range(const SpecTables<T> &S, T t) {
+  if (t < S.t_low_min) return 0;
+  if (t < S.t_mid_min) return t >= S.t_low_max ? 1 : -1;
+  return t >= S.t_high_max ? 2 : -1;
+}
+
+template <typename T>
+__device__ __forceinline__ T poly_cp(const T (&x)[6], T t) {
+  return x[0] + t * (x[1] + t * (x[2] + t * (x[3] + t * x[4])));
+}
+template <typename T>
+__device__ __forceinline__ T poly_h(const T (&x)[6], T t) {
+  return x[5] + t * (x[0] + t * (T(0.5) * x[1] + t * (T(1.0 / 3.0) * x[2] + t * (T(0.25) * x[3] + t * (T(0.2) * x[4])))));
 }
 
 template <typename T>
 __device__ __forceinline__ T nasa_h(const SpecTables<T> &S, const T *rec, int k, T t) {
-  T h, cp;
-  nasa_h_cp(S, rec, k, t, h, cp);
-  return h;
+  T x[6];
+  load_rec<T>(species_rec(S, rec, k, t), x);
+  return poly_h(x, t);
 }
 
 template <typename T>
 __device__ __forceinline__ T nasa_cp(const SpecTables<T> &S, const T *rec, int k, T t) {
-  const T tl = S.t_low[k];
-  const T te = t < tl ? tl : t;
-  T x[kRecLen];
-  load_rec<T>(rec + (2 * k + (t < S.t_mid[k] ? 0 : 1)) * kRecLen, x);
-  return (x[0] + te * (x[1] + te * (x[2] + te * (x[3] + te * x[4])))) * S.r_over_mw[k];
+  T x[6];
+  load_rec<T>(species_rec(S, rec, k, t), x);
+  return poly_cp(x, t);
+}
+
+// Coefficients of the mixture sum_k w_k (h_k, cp_k) at temperature t: the
+// species share the form of the polynomial, so their weighted coefficients
+// are summed (6 multiply-adds per species) and one polynomial is evaluated,
+// instead of two per species (about 20 operations each).  Where the species
+// lie in different ranges (r < 0) each record is chosen by itself.
+template <typename T, int NS>
+__device__ __forceinline__ void nasa_mix(const ChemParams &C, const T *rec, T t, int r, const T *w, T (&c)[6]) {
+  const SpecTables<T> &S = tab<T>(C);
+  constexpr int A = SpecCount<NS>::kArr;
+  const int ns = SpecCount<NS>::n(C);
+#pragma unroll
+  for (int q = 0; q < 6; ++q) c[q] = T(0);
+  if (r >= 0) {
+    const T *base = rec + r * kRecLen;
+#pragma unroll
+    for (int l = 0; l < A; ++l) {
+      if (l < ns) {
+        T x[6];
+        load_rec<T>(base + kRecRanges * kRecLen * l, x);
+#pragma unroll
+        for (int q = 0; q < 6; ++q) c[q] += w[l] * x[q];
+      }
+    }
+  } else {
+#pragma unroll
+    for (int l = 0; l < A; ++l) {
+      if (l < ns) {
+        T x[6];
+        load_rec<T>(species_rec(S, rec, l, t), x);
+#pragma unroll
+        for (int q = 0; q < 6; ++q) c[q] += w[l] * x[q];
+      }
+    }
+  }
 }
 
 template <typename T>
@@ -222,53 +269,34 @@ __device__ __forceinline__ void point_props(const ChemParams &C, const T *rec, T
 
 // Temperature from internal energy by Newton iteration (tolerance 1e-3 on
 // |1 - T1/T|, at most C.newton_max_iter iterations (1000 by default, as the
-// reference), warm start t), in the precision W:
-// FP64 for the plain and mixed paths, FP32 for the full-FP32 study.
-template <typename W, int NS>
-__device__ __forceinline__ W newton_temperature_w(const ChemParams &C, const W *rec, W e, const W *Y, W gas_const,
-                                                  W t, bool &capped) {
-  const SpecTables<W> &S = tab<W>(C);
-  constexpr int A = SpecCount<NS>::kArr;
-  const int ns = SpecCount<NS>::n(C);
-  W err = 1;
-  int iter = 0;
-  while (err > W(1e-3) && iter++ < C.newton_max_iter) {
-    W cp_tot = 0, h = 0;
-#pragma unroll
-    for (int l = 0; l < A; ++l) {
-      if (l < ns) {
-        W hl, cpl;
-        nasa_h_cp<W>(S, rec, l, t, hl, cpl);
-        cp_tot += cpl * Y[l];
-        h += hl * Y[l];
-      }
-    }
-    const W e_t = h - gas_const * t;
-    const W cvv = cp_tot - gas_const;
-    const W t1 = t - (e_t - e) / cvv;
-    err = fabs(W(1) - t1 / t);
+// reference), warm start t) in FP32, for the full-FP32 study; the FP64 Newton
+// of the other precisions is in point_finish.
+template <int NS>
+__device__ __forceinline__ float newton_temperature_f32(const ChemParams &C, const float *rec, float e, const float *Y,
+                                                        float gas_const, float t, bool &capped) {
+  float err = 1;
+  int iter = 0, range = -2;
+  float x[6];  // the mixture's coefficients, summed again only where t has left their range
+  while (err > 1e-3f && iter++ < C.newton_max_iter) {
+    const int r = common_range(C.f, t);
+    if (r != range || r < 0) nasa_mix<float, NS>(C, rec, t, r, Y, x), range = r;
+    const float t1 = t - (poly_h(x, t) - gas_const * t - e) / (poly_cp(x, t) - gas_const);
+    err = fabsf(1.0f - t1 / t);
     t = t1;
   }
-  capped = err > W(1e-3);
+  capped = err > 1e-3f;
   return t;
 }
 
-template <int NS>
-__device__ __forceinline__ double newton_temperature(const ChemParams &C, const double *rec, double e, const double *Y,
-                                                     double gas_const, double t, bool &capped) {
-  return newton_temperature_w<double, NS>(C, rec, e, Y, gas_const, t, capped);
+// 0.5 (sgn a + sgn b) min(|a|, |b|): the median of a, b and 0 in FP32 (four
+// min/max instructions); in FP64, whose comparisons run on the slow FP64
+// pipe, the smaller magnitude where the sign bits agree.
+__device__ __forceinline__ float minmod(float a, float b) {
+  return fmaxf(fminf(a, b), fminf(fmaxf(a, b), 0.0f));
 }
-
-template <typename T>
-__device__ __forceinline__ T sgn1(T a) {
-  return T((T(0) < a) - (a < T(0)));
-}
-
-// 0.5 (sgn a + sgn b) min(|a|, |b|), written as a sign test
-template <typename T>
-__device__ __forceinline__ T minmod(T a, T b) {
-  const T m = fmin(fabs(a), fabs(b));
-  return (a > T(0) && b > T(0)) ? m : ((a < T(0) && b < T(0)) ? -m : T(0));
+__device__ __forceinline__ double minmod(double a, double b) {
+  const double m = fmin(fabs(a), fabs(b));
+  return (__double2hiint(a) ^ __double2hiint(b)) < 0 ? 0.0 : copysign(m, a);
 }
 
 // AUSM+ pressure splitting P+(M) = (M+1)^2 (2-M)/4 + a M (M^2-1)^2 and
@@ -335,49 +363,57 @@ __device__ __forceinline__ void face_inviscid(const ChemParams &C, const T *rec,
   // L[4], R[4] hold the gauge pressure p - p_ref (p_ref = 0 in FP64)
   const T pref = T(C.p_ref);
   const T pl = L[4] + pref, pr = R[4] + pref;
+  // el, er: total enthalpy per unit mass, (rho E + p) / rho; c2l, c2r: gamma p / rho
   T el = T(0.5) * (L[1] * L[1] + L[2] * L[2] + L[3] * L[3]);
   T er = T(0.5) * (R[1] * R[1] + R[2] * R[2] + R[3] * R[3]);
-  T El, Er, gam_l, gam_r;
+  T c2l, c2r;
   if (NS == 0 || (NS < 0 && ns == 0)) {
-    El = el * L[0] + pl / T(kGammaAir - 1);
-    Er = er * R[0] + pr / T(kGammaAir - 1);
-    gam_l = gam_r = T(kGammaAir);
+    c2l = fdiv(T(kGammaAir) * pl, L[0]);
+    c2r = fdiv(T(kGammaAir) * pr, R[0]);
+    el += c2l * T(1.0 / (kGammaAir - 1));
+    er += c2r * T(1.0 / (kGammaAir - 1));
   } else {
     const SpecTables<T> &S = tab<T>(C);
-    T mwl = 0, mwr = 0;
+    T gas_l = 0, gas_r = 0;  // R_u / W
 #pragma unroll
     for (int l = 0; l < A; ++l)
-      if (l < ns) mwl += L[5 + l] * S.inv_mw[l], mwr += R[5 + l] * S.inv_mw[l];
-    const T t_l = fdiv(pl, L[0] * T(kRu) * mwl);
-    const T t_r = fdiv(pr, R[0] * T(kRu) * mwr);
-    T cpl = 0, cpr = 0, cvl = 0, cvr = 0;
+      if (l < ns) gas_l += L[5 + l] * S.cv_shift[l], gas_r += R[5 + l] * S.cv_shift[l];
+    const T t_l = fdiv(pl, L[0] * gas_l);
+    const T t_r = fdiv(pr, R[0] * gas_r);
+    T xl[6], xr[6];
+    const int rl = common_range(S, t_l), rr = common_range(S, t_r);
+    if (rl == rr && rl >= 0) {  // one load of each record serves both states
+      const T *base = rec + rl * kRecLen;
 #pragma unroll
-    for (int l = 0; l < A; ++l) {
-      if (l < ns) {
-        T hl, cl, hr, cr;
-        nasa_h_cp<T>(S, rec, l, t_l, hl, cl);
-        nasa_h_cp<T>(S, rec, l, t_r, hr, cr);
-        cpl += cl * L[5 + l];
-        cpr += cr * R[5 + l];
-        cvl += L[5 + l] * (cl - S.cv_shift[l]);
-        cvr += R[5 + l] * (cr - S.cv_shift[l]);
-        el += hl * L[5 + l];
-        er += hr * R[5 + l];
+      for (int q = 0; q < 6; ++q) xl[q] = xr[q] = T(0);
+#pragma unroll
+      for (int l = 0; l < A; ++l) {
+        if (l < ns) {
+          T x[6];
+          load_rec<T>(base + kRecRanges * kRecLen * l, x);
+#pragma unroll
+          for (int q = 0; q < 6; ++q) xl[q] += L[5 + l] * x[q], xr[q] += R[5 + l] * x[q];
+        }
       }
+    } else {
+      nasa_mix<T, NS>(C, rec, t_l, -1, L + 5, xl);
+      nasa_mix<T, NS>(C, rec, t_r, -1, R + 5, xr);
     }
-    El = L[0] * el - pl;
-    Er = R[0] * er - pr;
-    gam_l = fdiv(cpl, cvl);
-    gam_r = fdiv(cpr, cvr);
+    const T cpl = poly_cp(xl, t_l), cpr = poly_cp(xr, t_r);
+    el += poly_h(xl, t_l);
+    er += poly_h(xr, t_r);
+    c2l = fdiv(cpl, cpl - gas_l) * gas_l * t_l;
+    c2r = fdiv(cpr, cpr - gas_r) * gas_r * t_r;
   }
   const T alpha = T(3.0 / 16.0);
   const T k1 = k[0], k2 = k[1], k3 = k[2];
-  const T gk = fsqrt(k1 * k1 + k2 * k2 + k3 * k3);
-  const T igk = frcp(gk);
+  const T kk = k1 * k1 + k2 * k2 + k3 * k3;
+  const T igk = frsqrt(kk);
+  const T gk = kk * igk;
   const T ul = (k1 * L[1] + k2 * L[2] + k3 * L[3]) * igk;
   const T ur = (k1 * R[1] + k2 * R[2] + k3 * R[3]) * igk;
   const T rho_l = L[0], rho_r = R[0];
-  const T c = T(0.5) * (fsqrt(fdiv(gam_l * pl, rho_l)) + fsqrt(fdiv(gam_r * pr, rho_r)));
+  const T c = T(0.5) * (fsqrt(c2l) + fsqrt(c2r));
   const T ic = frcp(c);
   const T mach_l = ul * ic, mach_r = ur * ic;
   T mlp, mrn, plp, prn;
@@ -425,7 +461,7 @@ __device__ __forceinline__ void face_inviscid(const ChemParams &C, const T *rec,
   F[1] = coeff * (up ? L[1] : R[1]) + p_coeff * k1;
   F[2] = coeff * (up ? L[2] : R[2]) + p_coeff * k2;
   F[3] = coeff * (up ? L[3] : R[3]) + p_coeff * k3;
-  F[4] = up ? fdiv(coeff * (El + pl), rho_l) : fdiv(coeff * (Er + pr), rho_r);
+  F[4] = coeff * (up ? el : er);
 #pragma unroll
   for (int l = 0; l < A; ++l)
     if (l < ns) F[5 + l] = coeff * (up ? L[5 + l] : R[5 + l]);

@@ -62,30 +62,45 @@ __device__ __forceinline__ double local_time_step(const ChemParams &C, const T *
 
 // Stencil access of the primitives around one face (point p0 and its
 // neighbour p1 = p0 + e_d):  at(f, t) is field f at p0 + t e_d (t = -1..2);
-// cross(f, c, sg, t) is field f at p0 + t e_d + sg e_c.
-// The strides are scalars, not an array: an array indexed by the runtime
-// face direction would live in local memory and put a local load in front of
-// every stencil address.  c is a compile-time index after unrolling.
+// diff(f, 0) is its difference p1 - p0 along the normal, diff(f, 1) and
+// diff(f, 2) the sums over p0 and p1 of its two-sided differences along the
+// first and second tangential direction (tangent(d, 1), tangent(d, 2)), all
+// unscaled.  Strides and addresses are formed once per face from the runtime
+// direction, so that every access is one load at a fixed offset per field.
+__device__ __forceinline__ int tangent(int d, int q) { return q == 1 ? (d == 0 ? 1 : 0) : (d == 2 ? 1 : 2); }
+
 template <typename T>
 struct GlobalStencil {
   const T *__restrict__ P;
-  int N, p, sd, sj, sk;  // sd: stride along the face normal; sj, sk: strides of j and k
-  __device__ __forceinline__ int stride(int c) const { return c == 0 ? 1 : (c == 1 ? sj : sk); }
+  int N, p, sd, sa, sb;  // strides along the face normal and the tangential directions
+  __device__ __forceinline__ GlobalStencil(const T *P_, int N_, int p_, int d, int sj, int sk)
+      : P(P_), N(N_), p(p_), sd(d == 0 ? 1 : (d == 1 ? sj : sk)), sa(d == 0 ? sj : 1), sb(d == 2 ? sj : sk) {}
   __device__ __forceinline__ T at(int f, int t) const { return P[f * N + p + t * sd]; }
-  __device__ __forceinline__ T cross(int f, int c, int sg, int t) const {
-    return P[f * N + p + t * sd + sg * stride(c)];
+  __device__ __forceinline__ T diff(int f, int q) const {
+    if (q == 0) return at(f, 1) - at(f, 0);
+    const int o = f * N + p, s = q == 1 ? sa : sb;
+    return (P[o + s] - P[o - s]) + (P[o + sd + s] - P[o + sd - s]);
   }
 };
 
 // Face flux (inviscid minus viscous) of the face between p0 and p0 + e_d;
 // transport properties and geometry are read from the arenas at the global
 // point gp (and gp + gsd).
-// DIR >= 0 fixes the face direction at compile time (d_rt is then ignored).
-template <typename T, int NS, typename Stencil, int DIR = -1>
+//
+// Viscous part (ViscousScheme.cu:11-342, metrics averaged over both points).
+// Every flux is the physical flux dotted with the face vector k, so the
+// gradients enter as k . grad f = sum_r D_r a_r, with D_r the computational
+// derivative of f along r and a_r = grad xi_r . k: one dot product per field
+// instead of a 3 x 3 gradient, and no gradient kept for the species' second
+// pass.  The stress needs besides that k . (du/dx_c) = sum_r (k . D_r u)
+// grad xi_r and the divergence.  With the mixture polynomials of nasa_mix:
+// 128^3 mixed, face phase 0.705 -> 0.478 ms per stage (this form alone
+// 0.668), no spills in the TMA face kernel (468 bytes before); FP64 97 x 85
+// x 71, 0.576 -> 0.365 ms.
+template <typename T, int NS, typename Stencil>
 __device__ __forceinline__ void face_flux_gen(const ChemParams &C, const T *rec, const Stencil &S,
                                               const T *__restrict__ Pr, const T *__restrict__ G, int N, int gp, int gsd,
-                                              int d_rt, T *F) {
-  const int d = DIR >= 0 ? DIR : d_rt;
+                                              int d, T *F) {
   constexpr int A = SpecCount<NS>::kArr;
   const int ns = SpecCount<NS>::n(C);
   const int p = CCB_IDX(C, gp, N), p1 = CCB_IDX(C, gp + gsd, N);
@@ -116,92 +131,56 @@ __device__ __forceinline__ void face_flux_gen(const ChemParams &C, const T *rec,
   for (int l = 0; l < A; ++l)
     if (l < ns) D[l] = T(0.5) * (Pr[(2 + l) * N + p] + Pr[(2 + l) * N + p1]);
 
-  // ViscousScheme.cu:11-342, metrics averaged over both points (m and m1)
-  T met[3][3];
+  T a[3];                               // a_r, with the derivative's factor (1, 1/4, 1/4)
+  T n[3] = {T(0), T(0), T(0)};          // (k . grad) u_c
+  T t[3] = {T(0), T(0), T(0)};          // k . du/dx_c
+  T div = 0;
 #pragma unroll
-  for (int r = 0; r < 3; ++r)
+  for (int q = 0; q < 3; ++q) {
+    const int r = q == 0 ? d : tangent(d, q);
+    const T w = q == 0 ? T(0.5) : T(0.125);
+    T m[3], D3[3];
 #pragma unroll
-    for (int c = 0; c < 3; ++c) met[r][c] = T(0.5) * (G[(1 + 3 * r + c) * N + p] + G[(1 + 3 * r + c) * N + p1]);
-  auto deriv = [&](int f, T out[3]) {
+    for (int c = 0; c < 3; ++c) m[c] = w * (G[(1 + 3 * r + c) * N + p] + G[(1 + 3 * r + c) * N + p1]);
+    a[q] = m[0] * k[0] + m[1] * k[1] + m[2] * k[2];
 #pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      if (c == d)
-        out[c] = S.at(f, 1) - S.at(f, 0);
-      else
-        out[c] = T(0.25) * (S.cross(f, c, 1, 0) - S.cross(f, c, -1, 0) + S.cross(f, c, 1, 1) - S.cross(f, c, -1, 1));
-    }
-  };
-  auto grad = [&](const T dd[3], T g[3]) {
+    for (int c = 0; c < 3; ++c) D3[c] = S.diff(1 + c, q);
+    const T s = k[0] * D3[0] + k[1] * D3[1] + k[2] * D3[2];
 #pragma unroll
-    for (int c = 0; c < 3; ++c) g[c] = dd[0] * met[0][c] + dd[1] * met[1][c] + dd[2] * met[2][c];
-  };
-  T du[3], dv[3], dw[3], dT[3], gu[3], gv[3], gw[3], gT[3];
-  deriv(1, du);
-  deriv(2, dv);
-  deriv(3, dw);
-  deriv(5, dT);
-  grad(du, gu);
-  grad(dv, gv);
-  grad(dw, gw);
-  grad(dT, gT);
-  const T third = T(1.0 / 3.0);
-  const T txx = mu * (T(4) * gu[0] - T(2) * gv[1] - T(2) * gw[2]) * third;
-  const T tyy = mu * (T(4) * gv[1] - T(2) * gu[0] - T(2) * gw[2]) * third;
-  const T tzz = mu * (T(4) * gw[2] - T(2) * gu[0] - T(2) * gv[1]) * third;
-  const T txy = mu * (gu[1] + gv[0]);
-  const T txz = mu * (gu[2] + gw[0]);
-  const T tyz = mu * (gv[2] + gw[1]);
-  const T kx = k[0], ky = k[1], kz = k[2];
-  const T f1 = kx * txx + ky * txy + kz * txz;
-  const T f2 = kx * txy + ky * tyy + kz * tyz;
-  const T f3 = kx * txz + ky * tyz + kz * tzz;
-  const T um = T(0.5) * (S.at(1, 0) + S.at(1, 1));
-  const T vm = T(0.5) * (S.at(2, 0) + S.at(2, 1));
-  const T wm = T(0.5) * (S.at(3, 0) + S.at(3, 1));
-  T f4 = um * f1 + vm * f2 + wm * f3 + lam * (kx * gT[0] + ky * gT[1] + kz * gT[2]);
-  F[1] -= f1;
-  F[2] -= f2;
-  F[3] -= f3;
+    for (int c = 0; c < 3; ++c) n[c] += D3[c] * a[q], t[c] += s * m[c], div += D3[c] * m[c];
+  }
+  div *= T(2.0 / 3.0);
+  T f[3];
+#pragma unroll
+  for (int c = 0; c < 3; ++c) f[c] = mu * (n[c] + t[c] - div * k[c]);
+  auto normal_diff = [&](int fld) { return S.diff(fld, 0) * a[0] + S.diff(fld, 1) * a[1] + S.diff(fld, 2) * a[2]; };
+  T e = lam * normal_diff(5);
+#pragma unroll
+  for (int c = 0; c < 3; ++c) e += T(0.5) * (v[1][1 + c] + v[2][1 + c]) * f[c], F[1 + c] -= f[c];
   if (NS == 0 || (NS < 0 && ns == 0)) {
-    F[4] -= f4;
+    F[4] -= e;
     return;
   }
-  const SpecTables<T> &ST = tab<T>(C);
   const T tm = T(0.5) * (S.at(5, 0) + S.at(5, 1));
-  T gy[A][3];
-  T rho_uc = 0, rho_vc = 0, rho_wc = 0;
+  T total = 0;  // the correction velocity's flux: sum over the species' diffusive fluxes
 #pragma unroll
-  for (int l = 0; l < A; ++l) {
-    if (l < ns) {
-      T dy[3];
-      deriv(6 + l, dy);
-      grad(dy, gy[l]);
-      const T DMulH = D[l] * nasa_h<T>(ST, rec, l, tm);
-      f4 += kx * DMulH * gy[l][0];
-      f4 += ky * DMulH * gy[l][1];
-      f4 += kz * DMulH * gy[l][2];
-      rho_uc += D[l] * gy[l][0];
-      rho_vc += D[l] * gy[l][1];
-      rho_wc += D[l] * gy[l][2];
-    }
-  }
-  F[4] -= f4;
-  const T corr = kx * rho_uc + ky * rho_vc + kz * rho_wc;
+  for (int l = 0; l < A; ++l)
+    if (l < ns) D[l] *= normal_diff(6 + l), total += D[l];
+  T x[6];  // sum over the species of diffusive flux times enthalpy
+  nasa_mix<T, NS>(C, rec, tm, common_range(tab<T>(C), tm), D, x);
+  e += poly_h(x, tm);
+  F[4] -= e;
 #pragma unroll
-  for (int l = 0; l < A; ++l) {
-    if (l < ns) {
-      const T ym = T(0.5) * (S.at(6 + l, 0) + S.at(6 + l, 1));
-      F[5 + l] -= D[l] * (kx * gy[l][0] + ky * gy[l][1] + kz * gy[l][2]) - ym * corr;
-    }
-  }
+  for (int l = 0; l < A; ++l)
+    if (l < ns) F[5 + l] -= D[l] - T(0.5) * (v[1][5 + l] + v[2][5 + l]) * total;
 }
 
-template <typename T, int NS, int DIR = -1>
+template <typename T, int NS>
 __device__ __forceinline__ void face_flux(const ChemParams &C, const T *rec, const T *__restrict__ P,
                                           const T *__restrict__ Pr, const T *__restrict__ G, int N, int p, int d,
                                           int sd, int sj, int sk, T *F) {
-  GlobalStencil<T> S{P, N, p, sd, sj, sk};
-  face_flux_gen<T, NS, GlobalStencil<T>, DIR>(C, rec, S, Pr, G, N, p, sd, d, F);
+  const GlobalStencil<T> S(P, N, p, d, sj, sk);
+  face_flux_gen<T, NS>(C, rec, S, Pr, G, N, p, sd, d, F);
 }
 
 // gamma and acoustic speed of a point (Field.cu:187-200)
@@ -215,18 +194,14 @@ __device__ __forceinline__ void gamma_and_c(const ChemParams &C, const T *rec, T
     return;
   }
   const SpecTables<T> &S = tab<T>(C);
-  T mwi = 0, cp_tot = 0, cvv = 0;
+  T gas = 0, x[6];
 #pragma unroll
-  for (int l = 0; l < A; ++l) {
-    if (l < ns) {
-      const T cp = nasa_cp<T>(S, rec, l, temp);
-      mwi += Y[l] * S.inv_mw[l];
-      cp_tot += Y[l] * cp;
-      cvv += Y[l] * (cp - S.cv_shift[l]);
-    }
-  }
-  gamma = cp_tot / cvv;
-  c = sqrt(gamma * T(kRu) * temp * mwi);
+  for (int l = 0; l < A; ++l)
+    if (l < ns) gas += Y[l] * S.cv_shift[l];
+  nasa_mix<T, NS>(C, rec, temp, common_range(S, temp), Y, x);
+  const T cp = poly_cp(x, temp);
+  gamma = cp / (cp - gas);
+  c = sqrt(gamma * gas * temp);
 }
 
 // RK update of one interior point (TimeAdvanceFunc.cu:255-290 with the
@@ -266,7 +241,7 @@ __device__ __forceinline__ void point_finish(const ChemParams &C, const T *rec, 
   const double u = q[1] * inv, v = q[2] * inv, w = q[3] * inv;
   const double vel2 = u * u + v * v + w * w;
   double pres, temp;
-  double Yd[A];
+  T Yt[A];
   if (NS == 0 || (NS < 0 && ns == 0)) {
     pres = (kGammaAir - 1) * (q[4] - 0.5 * rho * vel2);
     temp = pres * kMwAir * inv / kRu;
@@ -274,23 +249,51 @@ __device__ __forceinline__ void point_finish(const ChemParams &C, const T *rec, 
     bool capped;
     double gas_const;
     if (!a.q32) {
-      double ysum = 0;
+      // The mixture's polynomial and gas constant are linear in the mass
+      // fractions, so they are summed over the partial densities q while
+      // these are in registers and scaled once by 1 / rho (and 1 / sum Y_k):
+      // the Newton keeps 7 values instead of the mass fractions.  Where an
+      // iterate leaves the range of the warm start, the sums are formed again
+      // from the partial densities just stored.
+      double x[6], gas = 0, qsum = 0;
 #pragma unroll
       for (int l = 0; l < A; ++l)
-        if (l < ns) Yd[l] = q[5 + l] * inv, ysum += Yd[l];
-      if (a.renorm_y) {
-        const double r = 1.0 / ysum;
-#pragma unroll
-        for (int l = 0; l < A; ++l)
-          if (l < ns) Yd[l] *= r;
-      }
-      double mwi = 0;
+        if (l < ns) gas += q[5 + l] * C.d.cv_shift[l], qsum += q[5 + l];
+      const double r = a.renorm_y ? 1.0 / qsum : inv;
+      int range = common_range(C.d, t_warm);
+      nasa_mix<double, NS>(C, rec_d, t_warm, range, q + 5, x);
 #pragma unroll
       for (int l = 0; l < A; ++l)
-        if (l < ns) mwi += Yd[l] * C.d.inv_mw[l];
-      gas_const = kRu * mwi;
+        if (l < ns) Yt[l] = T(q[5 + l] * r);
+#pragma unroll
+      for (int i = 0; i < 6; ++i) x[i] *= r;
+      gas_const = gas * r;
       const double e = q[4] * inv - 0.5 * vel2;
-      temp = newton_temperature<NS>(C, rec_d, e, Yd, gas_const, t_warm, capped);
+      double t = t_warm, err = 1;
+      int iter = 0;
+      while (err > 1e-3 && iter++ < C.newton_max_iter) {
+        if (iter > 1) {
+          const int now = common_range(C.d, t);
+          if (now != range || now < 0) {
+            range = now;
+#pragma unroll
+            for (int i = 0; i < 6; ++i) x[i] = 0;
+#pragma unroll 1
+            for (int l = 0; l < ns; ++l) {
+              const double w = a.Qout[(5 + l) * N + p] * r;
+              double y[6];
+              load_rec<double>(species_rec(C.d, rec_d, l, t), y);
+#pragma unroll
+              for (int i = 0; i < 6; ++i) x[i] += w * y[i];
+            }
+          }
+        }
+        const double t1 = t - (poly_h(x, t) - gas_const * t - e) / (poly_cp(x, t) - gas_const);
+        err = fabs(1.0 - t1 / t);
+        t = t1;
+      }
+      capped = err > 1e-3;
+      temp = t;
     } else {
       // full-FP32 study: Y, its renormalisation, e and the Newton in FP32
       // (only the FP32 bulk precision runs it; the FP64 instantiation reads
@@ -307,13 +310,12 @@ __device__ __forceinline__ void point_finish(const ChemParams &C, const T *rec, 
         for (int l = 0; l < A; ++l)
           if (l < ns) Yf[l] *= r;
       }
-      float mwi = 0;
+      float gcf = 0;
 #pragma unroll
       for (int l = 0; l < A; ++l)
-        if (l < ns) mwi += Yf[l] * C.f.inv_mw[l], Yd[l] = Yf[l];
-      const float gcf = float(kRu) * mwi;
+        if (l < ns) gcf += Yf[l] * C.f.cv_shift[l], Yt[l] = T(Yf[l]);
       const float ef = (float)q[4] * invf - 0.5f * (float)vel2;
-      temp = newton_temperature_w<float, NS>(C, rec_f32, ef, Yf, gcf, (float)t_warm, capped);
+      temp = newton_temperature_f32<NS>(C, rec_f32, ef, Yf, gcf, (float)t_warm, capped);
       gas_const = gcf;
     }
     if (capped) flags |= kStatusNewtonCap;
@@ -328,10 +330,9 @@ __device__ __forceinline__ void point_finish(const ChemParams &C, const T *rec, 
   Pn[3 * N + p] = T(w);
   Pn[4 * N + p] = T(pres - C.p_ref);  // gauge pressure
   Pn[5 * N + p] = T(temp);
-  T Yt[A];
 #pragma unroll
   for (int l = 0; l < A; ++l)
-    if (l < ns) Yt[l] = T(Yd[l]), Pn[(6 + l) * N + p] = Yt[l];
+    if (l < ns) Pn[(6 + l) * N + p] = Yt[l];
   if (a.closure) return;  // transport and the time step follow from the closure kernel
   T mu, lam, rd[A], gam, c;
   point_props<T, NS>(C, rec, T(temp), Yt, mu, lam, rd, gam, c);
@@ -345,7 +346,7 @@ __device__ __forceinline__ void point_finish(const ChemParams &C, const T *rec, 
     const double dtl = local_time_step<T>(C, G, N, p, rho, u, v, w, (double)c, (double)gam, (double)mu, three_d);
     dt_min = fmin(dt_min, dtl);
   }
-    }
+}
 
 template <typename T, int NS>
 __device__ __forceinline__ void point_update(const ChemParams &C, const T *rec, const double *rec_d,
@@ -424,8 +425,8 @@ template <typename T, int NS>
 struct StageSmem {
   static constexpr int A = SpecCount<NS>::kArr;
   static constexpr int NV = 5 + A;
-  static constexpr size_t kRecD = sizeof(double) * A * 2 * kRecLen;
-  static constexpr size_t kRecBytes = kRecD + (sizeof(T) == sizeof(double) ? 0 : sizeof(T) * A * 2 * kRecLen);
+  static constexpr size_t kRecD = sizeof(double) * A * kRecRanges * kRecLen;
+  static constexpr size_t kRecBytes = kRecD + (sizeof(T) == sizeof(double) ? 0 : sizeof(T) * A * kRecRanges * kRecLen);
   static constexpr size_t kBytes =
       kRecBytes + sizeof(T) * NV * (kTY * (kTX + 1) + (kTY + 1) * kTX + 2 * kTY * kTX);
   static_assert(kRecD % 16 == 0 && kRecBytes % 16 == 0, "records must stay 16-byte aligned");
@@ -441,7 +442,7 @@ __global__ void __launch_bounds__(kTX *kTY, sizeof(T) == 8 ? 1 : 2)
   extern __shared__ __align__(16) unsigned char smem_raw[];
   // NASA-7 records of both precisions (the bulk one for the face and point
   // thermodynamics, FP64 for the temperature Newton), then the face fluxes.
-  double *sRecD = reinterpret_cast<double *>(smem_raw);  // [A][2][kRecLen]
+  double *sRecD = reinterpret_cast<double *>(smem_raw);  // [A][kRecRanges][kRecLen]
   T *sRec = reinterpret_cast<T *>(smem_raw + (sizeof(T) == sizeof(double) ? 0 : StageSmem<T, NS>::kRecD));
   T *sFx = reinterpret_cast<T *>(smem_raw + StageSmem<T, NS>::kRecBytes);  // [NV][kTY][kTX+1]
   T *sFy = sFx + NV * kTY * (kTX + 1);                   // [NV][kTY+1][kTX]
@@ -464,7 +465,7 @@ __global__ void __launch_bounds__(kTX *kTY, sizeof(T) == 8 ? 1 : 2)
   T F[NV];
 
   {
-    const int tid = ty * kTX + tx, nrec = ns * 2 * kRecLen;
+    const int tid = ty * kTX + tx, nrec = ns * kRecRanges * kRecLen;
     const double *gd = param_rec<double>(C);
     const T *gt = param_rec<T>(C);
     for (int e = tid; e < nrec; e += kTX * kTY) {
@@ -590,14 +591,12 @@ template <int NS>
 __device__ __forceinline__ double total_energy(const ChemParams &C, double rho, double u, double v, double w, double p,
                                                double t, const double *Y) {
   const double *rec = param_rec<double>(C);
-  constexpr int A = SpecCount<NS>::kArr;
   const int ns = SpecCount<NS>::n(C);
   double e = 0.5 * rho * (u * u + v * v + w * w);
   if (NS == 0 || (NS < 0 && ns == 0)) return e + p / (kGammaAir - 1);
-#pragma unroll
-  for (int l = 0; l < A; ++l)
-    if (l < ns) e += nasa_h<double>(C.d, rec, l, t) * (rho * Y[l]);
-  return e - p;
+  double x[6];
+  nasa_mix<double, NS>(C, rec, t, common_range(C.d, t), Y, x);
+  return e + rho * poly_h(x, t) - p;
 }
 
 // Phase A: evaluate halo node e into its scratch slot.

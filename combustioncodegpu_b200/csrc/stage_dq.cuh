@@ -43,7 +43,7 @@ struct FacesDqLayout {
   static constexpr size_t kXch = round_up(sizeof(T) * kChunk * (TY - 1) * TX, 16);  // +y faces of rows 0..TY-2
   static constexpr size_t kYm = round_up(sizeof(T) * kNV * TX, 16);                 // -y boundary faces
   static constexpr size_t kXm = round_up(sizeof(T) * kNV * TY, 16);                 // -x boundary faces
-  static constexpr size_t kRec = round_up(sizeof(T) * A * 2 * kRecLen, 16);
+  static constexpr size_t kRec = round_up(sizeof(T) * A * kRecRanges * kRecLen, 16);
   // alignment slack + barriers + ring + exchange + boundary faces + NASA records
   static constexpr size_t kBytes = 128 + 128 + kRing * kPlaneBytes + kXch + kYm + kXm + kRec;
   static constexpr int kMinBlocks = TY == 4 ? 3 : (TY == 8 ? 2 : 1);
@@ -67,7 +67,7 @@ __global__ void __launch_bounds__(32 * TY, (FacesDqLayout<T, NS, TY, NCH>::kMinB
   T *sXm = reinterpret_cast<T *>(reinterpret_cast<unsigned char *>(sYm) + L::kYm);   // [NV][TY]
   T *sRec = reinterpret_cast<T *>(reinterpret_cast<unsigned char *>(sXm) + L::kXm);
   const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * TX + tx;
-  for (int e = tid, nrec = ns * 2 * kRecLen; e < nrec; e += TX * TY) sRec[e] = param_rec<T>(C)[e];
+  for (int e = tid, nrec = ns * kRecRanges * kRecLen; e < nrec; e += TX * TY) sRec[e] = param_rec<T>(C)[e];
   if (tid == 0) {
     for (int b = 0; b < L::kRing; ++b) mbar_init(&bars[b], 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -146,7 +146,7 @@ __global__ void __launch_bounds__(32 * TY, (FacesDqLayout<T, NS, TY, NCH>::kMinB
         doit = act, d = 1, sd = sj;
       }
       if (doit) {
-        Stencil S{plm, pl0, pl1, pl2, qq, d};
+        const Stencil S(plm, pl0, pl1, pl2, qq, d);
         face_flux_gen<T, NS>(C, sRec, S, a.Pr, a.G, N, gp, sd, d, F);
       } else {
 #pragma unroll

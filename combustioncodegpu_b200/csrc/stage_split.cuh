@@ -30,9 +30,9 @@ __global__ void __launch_bounds__(kTX *kTY, sizeof(T) == 8 ? 1 : 2)
   const int ns = SpecCount<NS>::n(C);
   const int nv = 5 + ns;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  T *sRec = reinterpret_cast<T *>(smem_raw);  // [A][2][kRecLen]
+  T *sRec = reinterpret_cast<T *>(smem_raw);  // [A][kRecRanges][kRecLen]
   const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * kTX + tx;
-  for (int e = tid, nrec = ns * 2 * kRecLen; e < nrec; e += kTX * kTY) sRec[e] = param_rec<T>(C)[e];
+  for (int e = tid, nrec = ns * kRecRanges * kRecLen; e < nrec; e += kTX * kTY) sRec[e] = param_rec<T>(C)[e];
   __syncthreads();  // the only barrier: threads may leave from here on
 
   const bool edge = (int)blockIdx.x >= a.n_regular;
@@ -94,10 +94,10 @@ __global__ void __launch_bounds__(256, MINB)
   const int ns = SpecCount<NS>::n(C);
   const int nv = 5 + ns;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  double *sRecD = reinterpret_cast<double *>(smem_raw);  // [A][2][kRecLen]
+  double *sRecD = reinterpret_cast<double *>(smem_raw);  // [A][kRecRanges][kRecLen]
   T *sRec = reinterpret_cast<T *>(smem_raw + (sizeof(T) == sizeof(double) ? 0 : StageSmem<T, NS>::kRecD));
   const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * UX + tx;
-  for (int e = tid, nrec = ns * 2 * kRecLen; e < nrec; e += UX * UY) {
+  for (int e = tid, nrec = ns * kRecRanges * kRecLen; e < nrec; e += UX * UY) {
     sRecD[e] = param_rec<double>(C)[e];
     if (sizeof(T) != sizeof(double)) sRec[e] = param_rec<T>(C)[e];
   }

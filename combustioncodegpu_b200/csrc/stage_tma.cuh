@@ -85,30 +85,37 @@ __device__ __forceinline__ void tma_load_plane(void *dst, const CUtensorMap *map
       : "memory");
 }
 
-// Primitives around one face from the plane ring: planes k-1 .. k+2 at
-// pm, p0, p1, p2; the face's first point at in-plane index q of plane k.
-// Scalar plane pointers (not an array): a runtime-indexed array would be
-// placed in local memory.  t and c are compile-time after unrolling; d is
-// the runtime face direction.
-template <typename T>
-struct SmemStencil {
-  const T *pm, *p0, *p1, *p2;
-  int q, d;
-  __device__ __forceinline__ const T *plane(int r) const {  // r = 0..3 -> k-1 .. k+2
-    return r == 0 ? pm : (r == 1 ? p0 : (r == 2 ? p1 : p2));
+// Primitives around one face from a ring of planes HX points wide with PV
+// values per field: planes k-1 .. k+2 at pm, p0, p1, p2, the face's first
+// point at in-plane index q of plane k, d its direction (runtime).  Holds the
+// in-plane addresses of the normal's four points and of the second tangential
+// direction's neighbours (the planes above and below unless d = 2).
+template <typename T, int HX, int PV>
+struct SmemStencilT {
+  const T *n0, *n1, *n2, *n3;  // p0 - e_d, p0, p0 + e_d, p0 + 2 e_d
+  const T *b0, *b1, *b2, *b3;  // p0 -+ e_b, p0 + e_d -+ e_b
+  int sa;                      // stride of the first tangential direction
+  __device__ __forceinline__ SmemStencilT(const T *pm, const T *p0, const T *p1, const T *p2, int q, int d) {
+    const int s = d == 0 ? 1 : HX;
+    const bool z = d == 2;
+    n1 = p0 + q;
+    n0 = z ? pm + q : n1 - s;
+    n2 = z ? p1 + q : n1 + s;
+    n3 = z ? p2 + q : n1 + 2 * s;
+    b0 = z ? n1 - HX : pm + q;
+    b1 = z ? n1 + HX : p1 + q;
+    b2 = z ? n2 - HX : pm + q + s;
+    b3 = z ? n2 + HX : p1 + q + s;
+    sa = d == 0 ? HX : 1;
   }
   __device__ __forceinline__ T at(int f, int t) const {
-    if (d == 2) return plane(1 + t)[f * kPlaneVals + q];
-    return p0[f * kPlaneVals + q + t * (d == 0 ? 1 : kHX)];
+    return (t == -1 ? n0 : (t == 0 ? n1 : (t == 1 ? n2 : n3)))[f * PV];
   }
-  __device__ __forceinline__ T cross(int f, int c, int sg, int t) const {
-    if (c == 2) {  // neighbour plane of the base point (k or k+t along z)
-      if (d == 2) return plane(1 + t + sg)[f * kPlaneVals + q];
-      return plane(1 + sg)[f * kPlaneVals + q + t * (d == 0 ? 1 : kHX)];
-    }
-    const int cs = sg * (c == 0 ? 1 : kHX);
-    if (d == 2) return plane(1 + t)[f * kPlaneVals + q + cs];
-    return p0[f * kPlaneVals + q + t * (d == 0 ? 1 : kHX) + cs];
+  __device__ __forceinline__ T diff(int f, int q) const {
+    const int o = f * PV;
+    if (q == 0) return n2[o] - n1[o];
+    if (q == 1) return ((n1 + sa)[o] - (n1 - sa)[o]) + ((n2 + sa)[o] - (n2 - sa)[o]);
+    return (b1[o] - b0[o]) + (b3[o] - b2[o]);
   }
 };
 
@@ -119,8 +126,8 @@ struct TmaLayout {
   static constexpr size_t kPlaneBytes = ((sizeof(T) * kNP * kPlaneVals + 127) / 128) * 128;
   static constexpr int XS = kTY * (kTX + 1), YS = (kTY + 1) * kTX, ZS = kTY * kTX;
   static constexpr size_t kFluxBytes = ((sizeof(T) * kNV * (XS + YS + 2 * ZS) + 15) / 16) * 16;
-  static constexpr size_t kRecD = sizeof(double) * SpecCount<NS>::kArr * 2 * kRecLen;
-  static constexpr size_t kRecBytes = kRecD + (sizeof(T) == sizeof(double) ? 0 : sizeof(T) * SpecCount<NS>::kArr * 2 * kRecLen);
+  static constexpr size_t kRecD = sizeof(double) * SpecCount<NS>::kArr * kRecRanges * kRecLen;
+  static constexpr size_t kRecBytes = kRecD + (sizeof(T) == sizeof(double) ? 0 : sizeof(T) * SpecCount<NS>::kArr * kRecRanges * kRecLen);
   // alignment slack + barriers + ring + fluxes + NASA records (FP64, bulk)
   static constexpr size_t kBytes = 128 + 128 + kSlots * kPlaneBytes + kFluxBytes + kRecBytes;
 };
@@ -166,7 +173,7 @@ __global__ void __launch_bounds__(kTX *kTY, 1)
   const int tx0 = t.i0 - 2 + B.g, ty0 = t.j0 - 2 + B.g;
   const int kfirst = t.k0 - 2, klast = t.k1 + 1;  // planes the sweep reads
 
-  for (int e = tid, nrec = ns * 2 * kRecLen; e < nrec; e += kTX * kTY) {
+  for (int e = tid, nrec = ns * kRecRanges * kRecLen; e < nrec; e += kTX * kTY) {
     sRecD[e] = param_rec<double>(C)[e];
     if (sizeof(T) != sizeof(double)) sRec[e] = param_rec<T>(C)[e];
   }
@@ -243,7 +250,7 @@ __global__ void __launch_bounds__(kTX *kTY, 1)
         gp = p - sj;
       }
       if (doit) {
-        SmemStencil<T> S{plm, pl0, pl1, pl2, qq, d};
+        const SmemStencilT<T, kHX, kPlaneVals> S(plm, pl0, pl1, pl2, qq, d);
         face_flux_gen<T, NS>(C, sRec, S, Pr, G, N, gp, sd, d, F);
 #pragma unroll
         for (int l = 0; l < NV; ++l)
@@ -328,31 +335,6 @@ __global__ void __launch_bounds__(kTX *kTY, 1)
 
 namespace ccb {
 
-// Primitives around one face from a ring of planes HX points wide with PV
-// values per field (the same access pattern as SmemStencil, for any tile
-// height).
-template <typename T, int HX, int PV>
-struct SmemStencilT {
-  const T *pm, *p0, *p1, *p2;
-  int q, d;
-  __device__ __forceinline__ const T *plane(int r) const {  // r = 0..3 -> k-1 .. k+2
-    return r == 0 ? pm : (r == 1 ? p0 : (r == 2 ? p1 : p2));
-  }
-  __device__ __forceinline__ T at(int f, int t) const {
-    if (d == 2) return plane(1 + t)[f * PV + q];
-    return p0[f * PV + q + t * (d == 0 ? 1 : HX)];
-  }
-  __device__ __forceinline__ T cross(int f, int c, int sg, int t) const {
-    if (c == 2) {
-      if (d == 2) return plane(1 + t + sg)[f * PV + q];
-      return plane(1 + sg)[f * PV + q + t * (d == 0 ? 1 : HX)];
-    }
-    const int cs = sg * (c == 0 ? 1 : HX);
-    if (d == 2) return plane(1 + t)[f * PV + q + cs];
-    return p0[f * PV + q + t * (d == 0 ? 1 : HX) + cs];
-  }
-};
-
 // Face kernel of the split stage with TMA-staged primitive planes: the
 // regular tiles of k_faces, each computing the +x, +y, +z faces of its points
 // from a ring of 4 planes (k-1 .. k+2) in shared memory; plane k+3 is
@@ -367,7 +349,7 @@ struct FacesTmaLayout {
   static constexpr int HX = TX + 4, HY = TY + 4, PV = HX * HY;
   static constexpr int kRing = 4;
   static constexpr size_t kPlaneBytes = ((sizeof(T) * (6 + SpecCount<NS>::kArr) * PV + 127) / 128) * 128;
-  static constexpr size_t kRec = ((sizeof(T) * SpecCount<NS>::kArr * 2 * kRecLen + 15) / 16) * 16;
+  static constexpr size_t kRec = ((sizeof(T) * SpecCount<NS>::kArr * kRecRanges * kRecLen + 15) / 16) * 16;
   // alignment slack + barriers + ring + NASA records
   static constexpr size_t kBytes = 128 + 128 + kRing * kPlaneBytes + kRec;
   // CTAs per SM that the shared memory allows (228 KB per SM, 1 KB reserved per CTA)
@@ -475,7 +457,7 @@ __device__ __forceinline__ int faces_tma_tile(const StageArgs<T> &a, const CUten
       for (int it = three_d ? 0 : 1; it < 3; ++it) {
         const int d = it == 0 ? 2 : it - 1;
         const int sd = d == 0 ? 1 : (d == 1 ? sj : sk);
-        SmemStencilT<T, L::HX, L::PV> S{plm, pl0, pl1, pl2, q, d};
+        const SmemStencilT<T, L::HX, L::PV> S(plm, pl0, pl1, pl2, q, d);
         face_flux_gen<T, NS>(C, sRec, S, a.Pr, a.G, N, p, sd, d, F);
 #pragma unroll
         for (int l = 0; l < NV; ++l)
@@ -517,7 +499,7 @@ __global__ void __launch_bounds__(TX *TY, (FacesTmaLayout<T, NS, TY, TX>::kMinBl
   T *sRec = reinterpret_cast<T *>(ring + L::kRing * L::kPlaneBytes);
   const int tid = threadIdx.y * TX + threadIdx.x;
   const Tile t = tiles[blockIdx.x];
-  for (int e = tid, nrec = ns * 2 * kRecLen; e < nrec; e += TX * TY) sRec[e] = param_rec<T>(C)[e];
+  for (int e = tid, nrec = ns * kRecRanges * kRecLen; e < nrec; e += TX * TY) sRec[e] = param_rec<T>(C)[e];
   if (tid == 0) {
     for (int b = 0; b < L::kRing; ++b) mbar_init(&bars[b], 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -544,7 +526,7 @@ __global__ void __launch_bounds__(TX *TY, (FacesTmaLayout<T, NS, TY, TX>::kMinBl
   T *sRec = reinterpret_cast<T *>(ring + L::kRing * L::kPlaneBytes);
   __shared__ int sh_tile;
   const int tid = threadIdx.y * TX + threadIdx.x;
-  for (int e = tid, nrec = ns * 2 * kRecLen; e < nrec; e += TX * TY) sRec[e] = param_rec<T>(C)[e];
+  for (int e = tid, nrec = ns * kRecRanges * kRecLen; e < nrec; e += TX * TY) sRec[e] = param_rec<T>(C)[e];
   if (tid == 0) {
     for (int b = 0; b < L::kRing; ++b) mbar_init(&bars[b], 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
