@@ -23,8 +23,9 @@ BUILD_BOUNDS = os.path.join(HERE, "_build_bounds")
 LIB_BOUNDS = os.path.join(HERE, "libcc_b200_bounds.so")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 SOURCES = [
+    "inst_d9.cu", "inst_f9.cu", "inst_dr16.cu", "inst_fr16.cu", "inst_dr11.cu", "inst_fr11.cu", "inst_dr8.cu",
+    "inst_fr8.cu", "inst_dr4.cu", "inst_fr4.cu", "inst_d0.cu", "inst_f0.cu",
     "api.cu", "misc.cu", "halo_plan.cpp", "noalloc.cu", "closure_train.cu",
-    "inst_d0.cu", "inst_d9.cu", "inst_dn.cu", "inst_f0.cu", "inst_f9.cu", "inst_fn.cu",
 ]
 
 

@@ -133,8 +133,8 @@ cudaError_t Launch<T, NS>::faces_tma_persistent(const StageArgs<T> &a, const Til
   const CUtensorMap *m = (const CUtensorMap *)maps;
   return with_face_shape(ty, tx, [&](auto ty_c, auto tx_c) -> cudaError_t {
     constexpr int TY = decltype(ty_c)::value, TX = decltype(tx_c)::value;
-    if constexpr (!FacesTmaLayout<T, NS, TY, TX>::kOk) {
-      return cudaErrorInvalidConfiguration;
+    if constexpr (NS < 0 || !FacesTmaLayout<T, NS, TY, TX>::kOk) {
+      return cudaErrorInvalidConfiguration;  // the persistent form: 0 or 9 species
     } else {
       static int per_sm = 0, n_sm = 0;  // CTAs per SM of this shape, SMs
       if (per_sm == 0) {
@@ -213,7 +213,7 @@ template <typename T, int NS>
 cudaError_t Launch<T, NS>::configure() {
   cudaError_t e = cudaFuncSetAttribute(k_stage<T, NS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)stage_smem());
   if (e != cudaSuccess) return e;
-  if (stage_tma_smem() <= 227 * 1024)
+  if constexpr (NS >= 0 && TmaLayout<T, NS>::kBytes <= 227 * 1024)
     e = cudaFuncSetAttribute(k_stage_tma<T, NS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)stage_tma_smem());
   for (const int sh : {0, 1, 2, 3, 4}) {  // every tile shape of the TMA face kernel whose ring fits
     const int ty = sh == 0 ? 4 : (sh == 1 || sh == 3 ? 8 : 16), tx = sh < 3 ? 32 : 16;
@@ -223,9 +223,10 @@ cudaError_t Launch<T, NS>::configure() {
         const int bytes = (int)FacesTmaLayout<T, NS, TY, TX>::kBytes;
         if (e == cudaSuccess)
           e = cudaFuncSetAttribute(k_faces_tma<T, NS, TY, TX>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-        if (e == cudaSuccess)
-          e = cudaFuncSetAttribute(k_faces_tma_persistent<T, NS, TY, TX>,
-                                   cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+        if constexpr (NS >= 0)
+          if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(k_faces_tma_persistent<T, NS, TY, TX>,
+                                     cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
       }
       return cudaSuccess;
     });
@@ -251,10 +252,13 @@ cudaError_t Launch<T, NS>::configure() {
 template <typename T, int NS>
 cudaError_t Launch<T, NS>::stage_tma(const StageArgs<T> &a, const void *maps, const ChemParams &C, int n_tiles,
                                      cudaStream_t s) {
-  if (n_tiles <= 0) return cudaSuccess;
-  if (stage_tma_smem() > 227 * 1024) return cudaErrorInvalidConfiguration;
-  k_stage_tma<T, NS><<<n_tiles, dim3(kTX, kTY), stage_tma_smem(), s>>>(a, (const CUtensorMap *)maps, C);
-  return cudaGetLastError();
+  if constexpr (NS < 0 || TmaLayout<T, NS>::kBytes > 227 * 1024) {
+    return cudaErrorInvalidConfiguration;  // 0 or 9 species, FP32 planes
+  } else {
+    if (n_tiles <= 0) return cudaSuccess;
+    k_stage_tma<T, NS><<<n_tiles, dim3(kTX, kTY), stage_tma_smem(), s>>>(a, (const CUtensorMap *)maps, C);
+    return cudaGetLastError();
+  }
 }
 
 template <typename T, int NS>

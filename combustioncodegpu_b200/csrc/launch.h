@@ -1,12 +1,18 @@
 // Host launchers of the templated kernels.  Each (precision, species count)
 // pair is instantiated in its own translation unit (inst_*.cu) so that the
-// large stage kernels compile in parallel.
+// large stage kernels compile in parallel: 0 and 9 species exactly, other
+// counts in classes of at most 4, 8, 11 and 16 (species_class), whose arrays
+// are sized for the class and whose loops stop at the count.
 #pragma once
 #include <cuda_runtime.h>
 
 #include "cc_common.h"
 
 namespace ccb {
+
+constexpr int species_class(int ns) {
+  return ns == 0 || ns == 9 ? ns : (ns <= 4 ? -4 : (ns <= 8 ? -8 : (ns <= 11 ? -11 : -16)));
+}
 
 template <typename T, int NS>
 struct Launch {
@@ -72,12 +78,11 @@ struct Launch {
 };
 
 #define CCB_DECLARE(T, NS) extern template struct Launch<T, NS>;
-CCB_DECLARE(double, 0)
-CCB_DECLARE(double, 9)
-CCB_DECLARE(double, -1)
-CCB_DECLARE(float, 0)
-CCB_DECLARE(float, 9)
-CCB_DECLARE(float, -1)
+#define CCB_DECLARE_COUNTS(T) \
+  CCB_DECLARE(T, 0) CCB_DECLARE(T, 9) CCB_DECLARE(T, -4) CCB_DECLARE(T, -8) CCB_DECLARE(T, -11) CCB_DECLARE(T, -16)
+CCB_DECLARE_COUNTS(double)
+CCB_DECLARE_COUNTS(float)
+#undef CCB_DECLARE_COUNTS
 #undef CCB_DECLARE
 
 // Non-templated helpers (misc.cu).

@@ -1,6 +1,6 @@
 // Device physics of the residual path, templated on the bulk precision T
 // (double for the plain path, float for the mixed path) and on the species
-// count NS (compile-time; -1 = runtime count up to kMaxSpec, 0 = perfect air).
+// count NS (n > 0: n species; -n: a runtime count of at most n; 0: perfect air).
 //
 // Reference counterparts (file:line in CombustionCodeGPU):
 //   NASA-7 h/cp with linear h below T_low ......... Thermo.cu:7-63
@@ -32,7 +32,7 @@ __device__ __forceinline__ const SpecTables<float> &tab<float>(const ChemParams 
 
 template <int NS>
 struct SpecCount {
-  static constexpr int kArr = NS > 0 ? NS : (NS == 0 ? 1 : kMaxSpec);
+  static constexpr int kArr = NS > 0 ? NS : (NS == 0 ? 1 : -NS);
   __device__ __forceinline__ static int n(const ChemParams &C) { return NS >= 0 ? NS : C.ns; }
 };
 

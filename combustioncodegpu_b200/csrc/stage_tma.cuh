@@ -354,7 +354,8 @@ struct FacesTmaLayout {
   static constexpr size_t kBytes = 128 + 128 + kRing * kPlaneBytes + kRec;
   // CTAs per SM that the shared memory allows (228 KB per SM, 1 KB reserved per CTA)
   static constexpr int kFit = (int)((228 * 1024) / (kBytes + 1024));
-  static constexpr bool kOk = kBytes <= 227 * 1024;
+  // built: the ring fits, and for the runtime counts the 32 x 4, 32 x 8 and 16 x 8 tiles only
+  static constexpr bool kOk = kBytes <= 227 * 1024 && (NS >= 0 || TX * TY <= 256);
   static constexpr int kMinBlocks = kFit < 1 ? 1 : (kFit > 3 ? 3 : kFit);
 };
 
