@@ -106,7 +106,9 @@ struct cc_ctx {
   int face_ty = 8;                // variants 3-5: tile height of the TMA face kernel (face_tx x face_ty x kz points)
   int face_tx = 32;               // variants 3-4: tile width of the TMA face kernel (32 or 16; 32 for variant 5)
   int force_tx = 0;               // cc_set_tile_width: face tile width, 0 = autotune
-  int update_occ = 0;             // 1: the FP32 update kernel sized for 4 CTAs per SM (autotuned)
+  int upd_form = 0;               // autotuned: 0 = k_update, 1 = the same sized for 4 CTAs per SM instead of 3 (FP32),
+                                  // 2 = k_update_tma
+  int upd_kz = 1;                 // k-planes per update tile
   int force_ty = 0;               // cc_set_tuning: face tile height, 0 = autotune
   std::vector<Tile> hutiles;      // variants 2-5: tiles of the update kernel (upd_tx x 256/upd_tx x kz)
   std::vector<int> ut_begin;      // per block: first update tile, + end
@@ -119,7 +121,7 @@ struct cc_ctx {
   std::vector<int> tile_begin, edge_begin;  // per block: first tile / edge tile (lists are block-ordered), + end
   bool per_block = false;         // cc_set_launch_mode: one launch per block per kernel instead of one per stage
   Tile *d_edges = nullptr;
-  void *faces = nullptr;          // split variant: face fluxes [3][n_var][N] (bulk precision)
+  void *faces = nullptr;          // split variant: face fluxes, grouped (store_faces; bulk precision)
   bool tma_ok = false;            // tensor maps built (the TMA variant can run)
   int force_variant = -1;         // cc_set_tuning: -1 autotune, else the variant
   int force_kz = 0;               // cc_set_tuning: k-planes per tile, 0 = autotune
@@ -130,6 +132,7 @@ struct cc_ctx {
   double *d_gcl = nullptr;        // [3][N] geometric term of the gauge-pressure momentum fluxes
   int kz = 1;                     // k-chunk of the stage tiles
   double tuned_ms = 0;            // stage-kernel time of the chosen configuration
+  CUtensorMap *d_qmaps = nullptr; // [2][2][n_blocks]: boxes of update tiles 32 x 8, 16 x 16 for Q[0], Q[1] per block
   CUtensorMap *d_tmaps = nullptr; // [3][2][n_blocks]: plane boxes of tile height 8, 4, 16 (kTmaRows) for the
                                   // primitive arenas P[0], P[1] per block
   unsigned *d_ticket = nullptr;   // tile counter of the persistent face kernel
@@ -383,6 +386,7 @@ void build_update_tiles(cc_ctx *c, int kz, int ux) {
   }
   c->ut_begin.push_back((int)c->hutiles.size());
   c->upd_tx = ux;
+  c->upd_kz = kz;
 }
 
 int upload_update_tiles(cc_ctx *c) {
@@ -485,7 +489,28 @@ int build_tensor_maps(cc_ctx *c) {
                           CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
       if (r != CUDA_SUCCESS) return fail(CC_ERR_CUDA, "cuTensorMapEncodeTiled failed (" + std::to_string((int)r) + ")");
     }
+  // the conserved state: one box per update tile (32 x 8, 16 x 16), all variables
+  std::vector<CUtensorMap> qmaps(2 * 2 * (size_t)nb);
+  for (int shape = 0; shape < 2; ++shape)
+    for (int buf = 0; buf < 2; ++buf)
+      for (int b = 0; b < nb; ++b) {
+        const HostBlock &h = c->blocks[b];
+        const cuuint64_t dims[4] = {(cuuint64_t)h.nx, (cuuint64_t)h.ny, (cuuint64_t)h.nz, (cuuint64_t)nv_of(c)};
+        const cuuint64_t strides[3] = {(cuuint64_t)h.nx * 8, (cuuint64_t)h.nx * h.ny * 8, (cuuint64_t)c->N * 8};
+        const cuuint32_t box[4] = {shape ? 16u : 32u, shape ? 16u : 8u, 1u, (cuuint32_t)nv_of(c)};
+        const cuuint32_t estr[4] = {1, 1, 1, 1};
+        CUresult r = encode(&qmaps[((size_t)shape * 2 + buf) * nb + b], CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 4,
+                            c->Q[buf] + h.off, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                            CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+        if (r != CUDA_SUCCESS)
+          return fail(CC_ERR_CUDA, "cuTensorMapEncodeTiled failed (" + std::to_string((int)r) + ")");
+      }
   void *p;
+  if (dev_alloc(c, &p, sizeof(CUtensorMap) * qmaps.size())) return CC_ERR_CUDA;
+  c->d_qmaps = (CUtensorMap *)p;
+  CK(cudaMemcpyAsync(c->d_qmaps, qmaps.data(), sizeof(CUtensorMap) * qmaps.size(), cudaMemcpyHostToDevice,
+                     c->stream));
   if (dev_alloc(c, &p, sizeof(CUtensorMap) * maps.size())) return CC_ERR_CUDA;
   c->d_tmaps = (CUtensorMap *)p;
   CK(cudaMemcpyAsync(c->d_tmaps, maps.data(), sizeof(CUtensorMap) * maps.size(), cudaMemcpyHostToDevice,
@@ -501,7 +526,7 @@ int build_tensor_maps(cc_ctx *c) {
 int apply_ownership(cc_ctx *c) {
   build_tiles_kz(c, c->kz);
   build_face_tiles(c, c->face_ty, c->kz, c->face_tx);
-  build_update_tiles(c, c->kz, c->upd_tx);
+  build_update_tiles(c, c->upd_kz, c->upd_tx);
   if (int r = upload_update_tiles(c)) return r;
   build_edge_tiles(c);
   c->hblocks_owned.clear();
@@ -609,8 +634,8 @@ int setup_device(cc_ctx *c) {
     if (dev_alloc(c, &p, sizeof(double) * N * nv_of(c))) return CC_ERR_CUDA;
     c->Q[b] = (double *)p;
   }
-  if (dev_alloc(c, &c->G, E * N * 10)) return CC_ERR_CUDA;
-  if (dev_alloc(c, &c->faces, E * N * 3 * nv_of(c))) return CC_ERR_CUDA;
+  if (dev_alloc(c, &c->G, E * N * (E == 4 ? 13 : 10))) return CC_ERR_CUDA;
+  if (dev_alloc(c, &c->faces, E * N * 3 * face_stride(nv_of(c), (int)E))) return CC_ERR_CUDA;
   if (dev_alloc(c, &p, sizeof(unsigned))) return CC_ERR_CUDA;
   c->d_ticket = (unsigned *)p;
   if (dev_alloc(c, &p, sizeof(GridBarrier))) return CC_ERR_CUDA;
@@ -705,7 +730,12 @@ int setup_device(cc_ctx *c) {
   CK(cudaMemsetAsync(c->stage64, 0, sizeof(double) * N * 10, c->stream));
   for (size_t b = 0; b < c->blocks.size(); ++b)
     if (int r = copy_fields_h2d(c, c->blocks[b], c->h_geo[b].data(), c->stage64, 10)) return r;
-  if (int r = from64(c, c->stage64, c->G, N * 10)) return r;
+  if (int r = dispatch(c, [&](auto tt, auto nn) -> int {
+        using T = typename decltype(tt)::type;
+        CK((Launch<T, decltype(nn)::value>::geometry(c->stage64, (T *)c->G, N, c->stream)));
+        return 0;
+      }))
+    return r;
   CK(cudaMemsetAsync(c->stage64, 0, sizeof(double) * N * std::max(np_of(c), 10), c->stream));
   return 0;
 }
@@ -948,7 +978,36 @@ int launch_stage(cc_ctx *c, StageArgs<T> a, int pc, int variant, int nt) {
 template <typename T, int NS>
 int launch_update(cc_ctx *c, StageArgs<T> a, const Tile *upd_tiles, int n_ut) {
   a.tiles = upd_tiles;
-  CK((Launch<T, NS>::update(a, c->chem, n_ut, c->stream, c->update_occ, c->upd_tx)));
+  if (c->upd_form == 2 && c->d_qmaps) {
+    const size_t nb = c->blocks.size();
+    const CUtensorMap *maps = c->d_qmaps + (c->upd_tx == 16 ? 2 * nb : 0);
+    CK((Launch<T, NS>::update_tma(a, maps + (a.Qin == c->Q[1] ? nb : 0), maps + (a.Qn == c->Q[1] ? nb : 0), c->chem,
+                                  n_ut, c->stream, c->upd_tx)));
+  } else {
+    CK((Launch<T, NS>::update(a, c->chem, n_ut, c->stream, c->upd_form == 1, c->upd_tx)));
+  }
+  return 0;
+}
+
+// The face kernels of the split variants (2-4): every face flux of the stage
+// into the face arena.
+template <typename T, int NS>
+int launch_faces(cc_ctx *c, StageArgs<T> a, int pc, int variant, int nt, int n_edge, const Tile *face_tiles,
+                 int n_ft) {
+  a.faces = (T *)c->faces;
+  if (!a.edge_tiles) a.edge_tiles = c->d_edges;
+  if (variant == 2) {
+    CK((Launch<T, NS>::faces(a, c->chem, nt, n_edge, c->stream)));
+    return 0;
+  }
+  // regular tiles from TMA-staged planes (persistent CTAs for 4), edge tiles through L1
+  const CUtensorMap *maps = c->d_tmaps + ((size_t)tma_shape(c->face_ty, c->face_tx) * 2 + pc) * c->blocks.size();
+  if (variant == 3)
+    CK((Launch<T, NS>::faces_tma(a, face_tiles, c->face_ty, c->face_tx, maps, c->chem, n_ft, c->stream)));
+  else
+    CK((Launch<T, NS>::faces_tma_persistent(a, face_tiles, c->face_ty, c->face_tx, maps, c->chem, n_ft, c->d_ticket,
+                                            c->stream)));
+  CK((Launch<T, NS>::faces(a, c->chem, 0, n_edge, c->stream)));
   return 0;
 }
 
@@ -957,38 +1016,25 @@ int launch_stage_range(cc_ctx *c, StageArgs<T> a, int pc, int variant, int nt, i
                        int n_ft, const Tile *upd_tiles, int n_ut) {
   if ((variant == 1 || variant == 3 || variant == 4 || variant == 5) && !c->d_tmaps)
     return fail(CC_ERR_STATE, "TMA variant without tensor maps");
+  if (variant == 0) {
+    CK((Launch<T, NS>::stage(a, c->chem, nt, c->stream)));
+    return 0;
+  }
+  if (variant == 1) {
+    CK((Launch<T, NS>::stage_tma(a, c->d_tmaps + (size_t)pc * c->blocks.size(), c->chem, nt, c->stream)));
+    return 0;
+  }
+  a.faces = (T *)c->faces;
   if (variant == 5) {  // faces differenced in the tile (dq), then the update
-    a.faces = (T *)c->faces;
     a.dq_direct = 1;
     const size_t nb = c->blocks.size();
     CK((Launch<T, NS>::faces_dq(a, face_tiles, c->d_tmaps + ((size_t)tma_shape(c->face_ty) * 2 + pc) * nb, c->chem,
                                 n_ft, c->face_ty, c->stream)));
-    if (int r = prof_event(c, c->ev_mid, c->ev_next_mid)) return r;
-    return launch_update<T, NS>(c, a, upd_tiles, n_ut);
+  } else if (int r = launch_faces<T, NS>(c, a, pc, variant, nt, n_edge, face_tiles, n_ft)) {
+    return r;
   }
-  if (variant == 1) {
-    CK((Launch<T, NS>::stage_tma(a, c->d_tmaps + (size_t)pc * c->blocks.size(), c->chem, nt, c->stream)));
-  } else if (variant == 2 || variant == 3 || variant == 4) {
-    a.faces = (T *)c->faces;
-    if (!a.edge_tiles) a.edge_tiles = c->d_edges;
-    if (variant == 2) {
-      CK((Launch<T, NS>::faces(a, c->chem, nt, n_edge, c->stream)));
-    } else {  // regular tiles from TMA-staged planes (persistent CTAs for 4), edge tiles through L1
-      const CUtensorMap *maps =
-          c->d_tmaps + ((size_t)tma_shape(c->face_ty, c->face_tx) * 2 + pc) * c->blocks.size();
-      if (variant == 3)
-        CK((Launch<T, NS>::faces_tma(a, face_tiles, c->face_ty, c->face_tx, maps, c->chem, n_ft, c->stream)));
-      else
-        CK((Launch<T, NS>::faces_tma_persistent(a, face_tiles, c->face_ty, c->face_tx, maps, c->chem, n_ft, c->d_ticket,
-                                                c->stream)));
-      CK((Launch<T, NS>::faces(a, c->chem, 0, n_edge, c->stream)));
-    }
-    if (int r = prof_event(c, c->ev_mid, c->ev_next_mid)) return r;
-    if (int r = launch_update<T, NS>(c, a, upd_tiles, n_ut)) return r;
-  } else {
-    CK((Launch<T, NS>::stage(a, c->chem, nt, c->stream)));
-  }
-  return 0;
+  if (int r = prof_event(c, c->ev_mid, c->ev_next_mid)) return r;
+  return launch_update<T, NS>(c, a, upd_tiles, n_ut);
 }
 
 // The closure transport of the new state (when on), the end of the stage's
@@ -1120,9 +1166,12 @@ int lusgs_alloc(cc_ctx *c) {
   return 0;
 }
 
-// Times the stage kernel of each candidate (kernel variant x k-chunk) on the
-// actual problem and keeps the fastest.  The candidates write only the
-// scratch halves of the ping-pong buffers, so the state is unchanged.
+// Times the candidates on the actual problem and keeps the fastest stage: the
+// fused variants as a whole (kernel x k-chunk); for the split variants the
+// face kernel (variant x tile x k-chunk) and the update kernel (form x tile x
+// k-chunk) each by itself, since neither's choice changes the other's time,
+// and their best as a whole.  The candidates write only the scratch halves of
+// the ping-pong buffers and the face arena, so the state is unchanged.
 template <typename T, int NS>
 int autotune(cc_ctx *c) {
   const char *env = std::getenv("CC_AUTOTUNE");
@@ -1153,10 +1202,6 @@ int autotune(cc_ctx *c) {
   cudaEvent_t e0, e1;
   CK(cudaEventCreate(&e0));
   CK(cudaEventCreate(&e1));
-  double best = 1e300;
-  int best_kz = c->kz;
-  int best_variant = 0;
-  int best_ty = c->face_ty, best_tx = c->face_tx;
   if (c->force_kz > 0) kzs.assign(1, c->force_kz);
   std::vector<int> variants;
   if (c->force_variant >= 0 && !variant_ok(c, c->force_variant))
@@ -1179,10 +1224,13 @@ int autotune(cc_ctx *c) {
         (Launch<T, NS>::faces_tma_smem(ty, 32) != 0 || Launch<T, NS>::faces_tma_smem(ty, 16) != 0))
       tys.push_back(ty);
   if (tys.empty()) return fail(CC_ERR_ARG, "the face tile height does not fit in shared memory in this precision");
-  std::vector<int> occs = c->precision == CC_FP64 ? std::vector<int>{0} : std::vector<int>{0, 1};
-  if (const char *oe = std::getenv("CC_UPDATE_OCC"))  // pins it (profiling runs, whose timings are distorted)
-    occs.assign(1, c->precision == CC_FP64 ? 0 : (oe[0] == '1' ? 1 : 0));
-  int best_occ = 0;
+  std::vector<int> forms{0};
+  if (c->precision != CC_FP64) forms.push_back(1);
+  if (c->d_qmaps) forms.push_back(2);
+  if (const char *oe = std::getenv("CC_UPDATE_OCC")) {  // pins it (profiling runs, whose timings are distorted)
+    const int form = std::atoi(oe);
+    forms.assign(1, std::count(forms.begin(), forms.end(), form) ? form : 0);
+  }
   // tile widths of the TMA face kernels: 32, and 16 (with heights 8 and 16)
   // for variants 3-4, whose narrower tiles waste fewer lanes on blocks whose
   // extent is not a multiple of 32
@@ -1197,54 +1245,102 @@ int autotune(cc_ctx *c) {
     if (v.empty() && (variant < 3 || variant > 4)) v.push_back(32);
     return v;
   };
+  // three launches of one candidate after one untimed: ms each
+  auto timed = [&](auto &&launch, double &ms) -> int {
+    if (int r = launch()) return r;
+    CK(cudaEventRecord(e0, c->stream));
+    for (int i = 0; i < 3; ++i)
+      if (int r = launch()) return r;
+    CK(cudaEventRecord(e1, c->stream));
+    CK(cudaEventSynchronize(e1));
+    float t = 0;
+    CK(cudaEventElapsedTime(&t, e0, e1));
+    ms = t / 3;
+    return 0;
+  };
+  auto set_tiles = [&](int kz, int ty, int tx) -> int {
+    build_tiles_kz(c, kz);
+    CK(cudaMemcpyAsync(c->d_tiles, c->htiles.data(), sizeof(Tile) * c->htiles.size(), cudaMemcpyHostToDevice,
+                       c->stream));
+    build_face_tiles(c, ty, kz, tx);
+    CK(cudaMemcpyAsync(c->d_ftiles, c->hftiles.data(), sizeof(Tile) * c->hftiles.size(), cudaMemcpyHostToDevice,
+                       c->stream));
+    return 0;
+  };
+  auto set_update_tiles = [&](int kz, int ux) -> int {
+    build_update_tiles(c, kz, ux);
+    return upload_update_tiles(c);
+  };
+  // the update kernel, with the step's-start state read as in two of three RK stages
+  double upd_ms = 0;
+  int upd_kz = c->kz, upd_tx = 32, upd_form = 0;
+  if (*std::max_element(variants.begin(), variants.end()) >= 2) {
+    upd_ms = 1e300;
+    std::vector<int> ukzs;
+    for (int kz : {1, 2, 4, 8, 16})
+      if (kz <= max_mz) ukzs.push_back(kz);
+    if (c->force_kz > 0) ukzs.assign(1, c->force_kz);
+    StageArgs<T> u = a;
+    u.faces = (T *)c->faces;
+    u.a = 0.75, u.b = 0.25;
+    for (int form : forms)
+      for (int ux : {32, 16})
+        for (int kz : ukzs) {
+          c->upd_form = form;
+          if (int r = set_update_tiles(kz, ux)) return r;
+          double ms = 0;
+          if (int r = timed([&] { return launch_update<T, NS>(c, u, c->d_utiles, (int)c->hutiles.size()); }, ms)) return r;
+          if (verbose)
+            std::fprintf(stderr, "cc autotune: update form %d tile %dx%dx%d %.4f ms\n", form, ux, 256 / ux, kz, ms);
+          if (ms < upd_ms) upd_ms = ms, upd_kz = kz, upd_tx = ux, upd_form = form;
+        }
+  }
+  c->upd_form = upd_form;
+  if (int r = set_update_tiles(upd_kz, upd_tx)) return r;
+  // the best split configuration by the sum of its two kernels, the best of
+  // the others as a whole; then the split one as a whole too
+  a.a = 0.75, a.b = 0.25;
+  struct Best {
+    double ms = 1e300;
+    int variant = 0, kz = 1, ty = 8, tx = 32;
+  } split, whole;
+  auto launch_whole = [&](int variant) {
+    return launch_stage_range<T, NS>(c, a, pc, variant, (int)c->htiles.size(), (int)c->hedges.size(), c->d_ftiles,
+                                     (int)c->hftiles.size(), c->d_utiles, (int)c->hutiles.size());
+  };
   for (int variant : variants) {
+    const bool is_split = variant >= 2 && variant <= 4;
     for (int ty : (variant >= 3 ? tys : std::vector<int>{8})) {
       for (int tx : txs_of(variant, ty)) {
-      for (int occ : (variant >= 2 ? occs : std::vector<int>{0})) {
-      c->update_occ = occ;
-      for (int kz : kzs) {
-        build_tiles_kz(c, kz);
-        CK(cudaMemcpyAsync(c->d_tiles, c->htiles.data(), sizeof(Tile) * c->htiles.size(), cudaMemcpyHostToDevice,
-                           c->stream));
-        build_face_tiles(c, ty, kz, tx);
-        CK(cudaMemcpyAsync(c->d_ftiles, c->hftiles.data(), sizeof(Tile) * c->hftiles.size(), cudaMemcpyHostToDevice,
-                           c->stream));
-        build_update_tiles(c, kz, variant == 3 || variant == 4 ? tx : 32);
-        if (int r = upload_update_tiles(c)) return r;
-        const int nt = (int)c->htiles.size();
-        if (int r = launch_stage<T, NS>(c, a, pc, variant, nt)) return r;
-        CK(cudaEventRecord(e0, c->stream));
-        for (int r = 0; r < 3; ++r)
-          if (int rr = launch_stage<T, NS>(c, a, pc, variant, nt)) return rr;
-        CK(cudaEventRecord(e1, c->stream));
-        CK(cudaEventSynchronize(e1));
-        float ms = 0;
-        CK(cudaEventElapsedTime(&ms, e0, e1));
-        if (verbose)
-          std::fprintf(stderr, "cc autotune: %s tile %dx%dx%d update-occ %d tiles=%d %.4f ms\n",
-                       kVariantName[variant], variant >= 3 ? tx : kTX, variant >= 3 ? ty : kTY, kz, occ,
-                       variant >= 3 ? (int)c->hftiles.size() : nt, ms / 3);
-        if (ms / 3 < best)
-          best = ms / 3, best_kz = kz, best_variant = variant, best_ty = ty, best_tx = tx, best_occ = occ;
-      }
-      }
+        for (int kz : kzs) {
+          if (int r = set_tiles(kz, ty, tx)) return r;
+          const int nt = (int)c->htiles.size(), n_edge = (int)c->hedges.size(), n_ft = (int)c->hftiles.size();
+          double ms = 0;
+          auto launch = [&] {
+            return is_split ? launch_faces<T, NS>(c, a, pc, variant, nt, n_edge, c->d_ftiles, n_ft) : launch_whole(variant);
+          };
+          if (int r = timed(launch, ms)) return r;
+          if (is_split) ms += upd_ms;
+          if (verbose)
+            std::fprintf(stderr, "cc autotune: %s tile %dx%dx%d tiles=%d %.4f ms\n", kVariantName[variant],
+                         variant >= 3 ? tx : kTX, variant >= 3 ? ty : kTY, kz, variant >= 3 ? n_ft : nt, ms);
+          Best &best = is_split ? split : whole;
+          if (ms < best.ms) best = Best{ms, variant, kz, ty, tx};
+        }
       }
     }
   }
-  c->update_occ = best_occ;
+  if (split.ms < 1e300) {
+    if (int r = set_tiles(split.kz, split.ty, split.tx)) return r;
+    if (int r = timed([&] { return launch_whole(split.variant); }, split.ms)) return r;
+  }
+  const Best best = split.ms < whole.ms ? split : whole;
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
-  if (best == 1e300) return fail(CC_ERR_ARG, "the face tile does not fit in shared memory in this precision");
-  build_tiles_kz(c, best_kz);
-  CK(cudaMemcpyAsync(c->d_tiles, c->htiles.data(), sizeof(Tile) * c->htiles.size(), cudaMemcpyHostToDevice,
-                     c->stream));
-  build_face_tiles(c, best_variant >= 3 ? best_ty : 8, best_kz, best_variant >= 3 ? best_tx : 32);
-  CK(cudaMemcpyAsync(c->d_ftiles, c->hftiles.data(), sizeof(Tile) * c->hftiles.size(), cudaMemcpyHostToDevice,
-                     c->stream));
-  build_update_tiles(c, best_kz, best_variant == 3 || best_variant == 4 ? best_tx : 32);
-  if (int r = upload_update_tiles(c)) return r;
-  c->variant = best_variant;
-  c->tuned_ms = best;
+  if (best.ms == 1e300) return fail(CC_ERR_ARG, "the face tile does not fit in shared memory in this precision");
+  if (int r = set_tiles(best.kz, best.variant >= 3 ? best.ty : 8, best.variant >= 3 ? best.tx : 32)) return r;
+  c->variant = best.variant;
+  c->tuned_ms = best.ms;
   CK(cudaMemsetAsync(c->d_status, 0, sizeof(unsigned), c->stream));
   CK(cudaStreamSynchronize(c->stream));
   return 0;

@@ -92,6 +92,13 @@ struct ClosureDev {
                                         // run-time check (points of the tiles it sent back)
 };
 
+// Values per point and direction of the face arena (stage.cuh, store_faces):
+// FP64 one by one; FP32 in groups of four, the last of two where at most two
+// are left.
+CCB_HD constexpr int face_stride(int nv, int elem) {
+  return elem == 8 ? nv : nv / 4 * 4 + (nv % 4 == 0 ? 0 : (nv % 4 <= 2 ? 2 : 4));
+}
+
 // One block of the multiblock grid in the concatenated field arena.
 struct BlockInfo {
   int mx, my, mz, g;
@@ -201,7 +208,7 @@ struct StageArgs {
   int q32;                   // 1: full-FP32 precision (conserved variables rounded to FP32, FP32 Newton)
   int closure;               // 1: transport of the new state comes from the learned closure kernel (not here)
   const double *gcl;         // [3][N]: sum over directions of k(+) - k(-) per point (p_ref != 0), else null
-  // split variant (stage_split.cuh): face fluxes [3][n_var][N] (face d of
+  // split variant (stage_split.cuh): face fluxes (store_faces; face d of
   // point p lies between p and p + e_d), the tiles of the minus-side face
   // layers (i, j or k = -1; direction in Tile::pad0), regular tile count
   T *faces;

@@ -7,6 +7,7 @@
 #include "stage.cuh"
 #include "stage_tma.cuh"
 #include "stage_split.cuh"
+#include "stage_update.cuh"
 #include "stage_dq.cuh"
 #include "closure.cuh"
 #include "lusgs.cuh"
@@ -177,6 +178,20 @@ cudaError_t Launch<T, NS>::update(const StageArgs<T> &a, const ChemParams &C, in
 }
 
 template <typename T, int NS>
+cudaError_t Launch<T, NS>::update_tma(const StageArgs<T> &a, const void *maps_in, const void *maps_n,
+                                      const ChemParams &C, int n_tiles, cudaStream_t s, int ux) {
+  if (n_tiles <= 0) return cudaSuccess;
+  if (ux != 32 && ux != 16) return cudaErrorInvalidValue;
+  const CUtensorMap *mi = (const CUtensorMap *)maps_in, *mn = (const CUtensorMap *)maps_n;
+  constexpr size_t smem = UpdateTmaLayout<T, NS>::kBytes;
+  if (ux == 32)
+    k_update_tma<T, NS, 32><<<n_tiles, dim3(32, 8), smem, s>>>(a, mi, mn, C);
+  else
+    k_update_tma<T, NS, 16><<<n_tiles, dim3(16, 16), smem, s>>>(a, mi, mn, C);
+  return cudaGetLastError();
+}
+
+template <typename T, int NS>
 cudaError_t Launch<T, NS>::props_mlp(const T *P, T *Pr, int64_t N, const void *cl, unsigned *status,
                                      const ChemParams &C, cudaStream_t s) {
   if constexpr (NS == 0) {
@@ -196,6 +211,12 @@ cudaError_t Launch<T, NS>::props_mlp(const T *P, T *Pr, int64_t N, const void *c
     k_props_mlp<T, NS><<<grid, kMlpRows, kMlpSmem, s>>>(P, Pr, N, *static_cast<const ClosureDev *>(cl), status, C);
     return cudaGetLastError();
   }
+}
+
+template <typename T, int NS>
+cudaError_t Launch<T, NS>::geometry(const double *src, T *G, int64_t N, cudaStream_t s) {
+  k_geometry<T><<<(unsigned)((N + 255) / 256), 256, 0, s>>>(src, G, N);
+  return cudaGetLastError();
 }
 
 template <typename T, int NS>
@@ -231,6 +252,11 @@ cudaError_t Launch<T, NS>::configure() {
       return cudaSuccess;
     });
   }
+  constexpr int upd = (int)UpdateTmaLayout<T, NS>::kBytes;
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(k_update_tma<T, NS, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, upd);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(k_update_tma<T, NS, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize, upd);
   if constexpr (NS != 0) {  // the closure kernel (set here too, before any stream capture)
     if (e == cudaSuccess)
       e = cudaFuncSetAttribute(k_props_mlp<T, NS>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMlpSmem);

@@ -31,6 +31,11 @@ struct Launch {
   // ux: tile width, 32 (32 x 8 tiles) or 16 (16 x 16)
   static cudaError_t update(const StageArgs<T> &a, const ChemParams &C, int n_tiles, cudaStream_t s,
                             int high_occ = 0, int ux = 32);
+  // update kernel with the conserved states staged by TMA (stage_update.cuh);
+  // maps_in, maps_n = per block the boxes of a.Qin and a.Qn for tiles of width
+  // ux
+  static cudaError_t update_tma(const StageArgs<T> &a, const void *maps_in, const void *maps_n, const ChemParams &C,
+                                int n_tiles, cudaStream_t s, int ux);
   // split variant with TMA-staged planes in the face kernel: tiles of tx x ty
   // points (32 x 4, 32 x 8, 32 x 16, 16 x 8, 16 x 16; the x 16 shapes in FP32
   // only), smem 0 when the ring does not fit
@@ -49,6 +54,8 @@ struct Launch {
   // learned transport closure (closure.cuh) over every arena point; cl is a ClosureDev
   static cudaError_t props_mlp(const T *P, T *Pr, int64_t N, const void *cl, unsigned *status, const ChemParams &C,
                                cudaStream_t s);
+  // geometry arena (k_geometry) from [10][N] FP64 fields
+  static cudaError_t geometry(const double *src, T *G, int64_t N, cudaStream_t s);
   // geometric term of the gauge-pressure momentum fluxes (k_gcl)
   static cudaError_t gcl(const BlockInfo *blocks, int nblocks, const T *G, int64_t N, int64_t n_interior,
                          double *out, cudaStream_t s);

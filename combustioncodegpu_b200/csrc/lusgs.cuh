@@ -106,8 +106,22 @@ __global__ void __launch_bounds__(kTX *kTY, sizeof(T) == 8 ? 1 : 2) k_lusgs_rhs(
   const T *__restrict__ P = a.P;
   const T *__restrict__ G = a.G;
   const T *__restrict__ Fx = a.faces;
-  const T *__restrict__ Fy = a.faces + (size_t)nv * N;
-  const T *__restrict__ Fz = a.faces + (size_t)2 * nv * N;
+  const T *__restrict__ Fy = a.faces + (size_t)face_stride(nv, (int)sizeof(T)) * N;
+  const T *__restrict__ Fz = a.faces + (size_t)2 * face_stride(nv, (int)sizeof(T)) * N;
+  // the residual of the variables of face group g at point p
+  constexpr int W = kFaceGroup<T>;
+  auto residual_group = [&](int p, int g, double (&dq)[W]) {
+    T acc[W];
+    face_sum<T>(Fx, Fy, Fz, N, nv, g, p, p - 1, p - sj, three_d ? p - sk : p, acc);
+#pragma unroll
+    for (int i = 0; i < W; ++i) {
+      const int l = W * g + i;
+      dq[i] = 0.0;
+      if (l >= nv) continue;
+      dq[i] = -(double)acc[i];
+      if (a.gcl && l >= 1 && l <= 3) dq[i] -= C.p_ref * a.gcl[(l - 1) * N + p];
+    }
+  };
   const T *rec = param_rec<T>(C);
   const int col = (int)B.base + (act ? i + sj * j : 0);
   for (int k = t.k0; k < t.k1; ++k) {
@@ -121,7 +135,13 @@ __global__ void __launch_bounds__(kTX *kTY, sizeof(T) == 8 ? 1 : 2) k_lusgs_rhs(
 #pragma unroll
     for (int f = 0; f < 6 + A; ++f) pv[f] = (act && f < 6 + ns) ? P[f * N + p] : T(0);
 #pragma unroll
-    for (int r = 0; r < 10; ++r) gv[r] = act ? G[r * N + p] : T(0);
+    for (int d = 0; d < 3; ++d) {
+      GeoRow<T> g{};
+      if (act) g = geo_row(G, N, d, p);
+      gv[0] = g.J;
+#pragma unroll
+      for (int c = 0; c < 3; ++c) gv[1 + 3 * d + c] = g.m[c];
+    }
     if (act) mu_t = a.Pr[p];
     double qc[4];
 #pragma unroll
@@ -129,33 +149,28 @@ __global__ void __launch_bounds__(kTX *kTY, sizeof(T) == 8 ? 1 : 2) k_lusgs_rhs(
     if (NV > 16) {  // runtime species count beyond 11: plain stores of the wider rows
       if (act) {
 #pragma unroll
-        for (int l = 0; l < NV; ++l) {
-          if (l < nv) {
-            const int o = l * N + p;
-            T acc = Fx[o] - Fx[o - 1];
-            acc += Fy[o] - Fy[o - sj];
-            if (three_d) acc += Fz[o] - Fz[o - sk];
-            double dq = -(double)acc;
-            if (a.gcl && l >= 1 && l <= 3) dq -= C.p_ref * a.gcl[(l - 1) * N + p];
-            L.R[sp * lp + l] = dq;
-            L.Qs[sp * lp + l] = a.Qin[o];
+        for (int g = 0; g < kFaceGroups<T, NV>; ++g) {
+          if (W * g >= nv) continue;
+          double dq[W];
+          residual_group(p, g, dq);
+#pragma unroll
+          for (int i = 0; i < W; ++i) {
+            const int l = W * g + i;
+            if (l < nv) L.R[sp * lp + l] = dq[i], L.Qs[sp * lp + l] = a.Qin[l * N + p];
           }
         }
       }
     } else {
       double rv[16], qv[16];
 #pragma unroll
-      for (int l = 0; l < 16; ++l) {
-        rv[l] = qv[l] = 0.0;
-        if (act && l < nv) {
-          const int o = l * N + p;
-          T acc = Fx[o] - Fx[o - 1];
-          acc += Fy[o] - Fy[o - sj];
-          if (three_d) acc += Fz[o] - Fz[o - sk];
-          double dq = -(double)acc;
-          if (a.gcl && l >= 1 && l <= 3) dq -= C.p_ref * a.gcl[(l - 1) * N + p];
-          rv[l] = dq;
-          qv[l] = a.Qin[o];
+      for (int g = 0; g < 16 / W; ++g) {
+        double dq[W] = {};
+        if (act && W * g < nv) residual_group(p, g, dq);
+#pragma unroll
+        for (int i = 0; i < W; ++i) {
+          const int l = W * g + i;
+          rv[l] = dq[i];
+          qv[l] = act && l < nv ? a.Qin[l * N + p] : 0.0;
         }
       }
       lusgs_put_rows(buf, rv, lp == 16 ? sp : -1, L.R, 16);
@@ -393,7 +408,7 @@ __global__ void __launch_bounds__(kTX *kTY) k_lusgs_update(const StageArgs<T> a,
 #pragma unroll
       for (int l = 0; l < NV; ++l)
         if (l < nv) dq[l] = L.R[sp * L.lp + l];
-      point_update<T, NS>(C, sRec, sRecD, a, p, N, dq, (double)a.G[p], (double)a.P[5 * N + p], three_d, flags,
+      point_update<T, NS>(C, sRec, sRecD, a, p, N, dq, (double)geo_jac(a.G, N, p), (double)a.P[5 * N + p], three_d, flags,
                           dt_min);
     }
   }

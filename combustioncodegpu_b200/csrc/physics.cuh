@@ -40,11 +40,22 @@ struct SpecCount {
 // in FP64 (the plain path), hardware approximations in FP32 (the mixed path;
 // relative error of a few ulp, far below the path's 1e-5 error budget).
 __device__ __forceinline__ double fdiv(double a, double b) { return a / b; }
-__device__ __forceinline__ float fdiv(float a, float b) { return __fdividef(a, b); }
+// (The approximations flush denormal operands, which saves their scaling
+// instructions: the values they are taken of, states, viscosities and sums of
+// mole fractions, are far from 1e-38.)
 __device__ __forceinline__ double frcp(double a) { return 1.0 / a; }
-__device__ __forceinline__ float frcp(float a) { return __fdividef(1.0f, a); }
+__device__ __forceinline__ float frcp(float a) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a));
+  return r;
+}
+__device__ __forceinline__ float fdiv(float a, float b) { return a * frcp(b); }
 __device__ __forceinline__ double fsqrt(double a) { return sqrt(a); }
-__device__ __forceinline__ float fsqrt(float a) { return a * rsqrtf(a); }
+__device__ __forceinline__ float fsqrt(float a) {
+  float r;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a));
+  return a * r;
+}
 __device__ __forceinline__ double frsqrt(double a) { return rsqrt(a); }
 __device__ __forceinline__ float frsqrt(float a) { return rsqrtf(a); }
 
@@ -174,7 +185,10 @@ __device__ __forceinline__ double pow_m0145<double>(double x) {
 }
 template <>
 __device__ __forceinline__ float pow_m0145<float>(float x) {
-  return __powf(x, -0.145f);
+  float l, r;
+  asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(l) : "f"(x));
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(-0.145f * l));
+  return r;
 }
 
 // Wilke mixture viscosity, modified-Wilke conductivity and constant-Schmidt
@@ -250,21 +264,17 @@ __device__ __forceinline__ void point_props(const ChemParams &C, const T *rec, T
     return;
   }
   const SpecTables<T> &S = tab<T>(C);
-  T cp[A];
-  T mwi = 0, cp_tot = 0, cvv = 0;
+  T cp[A], mwi = 0, cp_mix = 0;
 #pragma unroll
-  for (int l = 0; l < A; ++l) {
-    if (l < ns) {
-      cp[l] = nasa_cp<T>(S, rec, l, temp);
-      mwi += Y[l] * S.inv_mw[l];
-      cp_tot += Y[l] * cp[l];
-      cvv += Y[l] * (cp[l] - S.cv_shift[l]);
-    }
-  }
-  const T mw = frcp(mwi);
-  gamma = fdiv(cp_tot, cvv);
-  c = fsqrt(gamma * T(kRu) * temp * mwi);
-  transport<T, NS>(C, temp, Y, mw, cp, mu, lam, rhod);
+  for (int l = 0; l < A; ++l)
+    if (l < ns) cp[l] = nasa_cp<T>(S, rec, l, temp);
+#pragma unroll
+  for (int l = 0; l < A; ++l)
+    if (l < ns) mwi += Y[l] * S.inv_mw[l], cp_mix += Y[l] * cp[l];
+  const T gas = T(kRu) * mwi;
+  gamma = fdiv(cp_mix, cp_mix - gas);
+  c = fsqrt(gamma * gas * temp);
+  transport<T, NS>(C, temp, Y, frcp(mwi), cp, mu, lam, rhod);
 }
 
 // Temperature from internal energy by Newton iteration (tolerance 1e-3 on
@@ -340,8 +350,6 @@ __device__ __forceinline__ void face_inviscid(const ChemParams &C, const T *rec,
   const int nv = 5 + ns;
   T L[NV], R[NV];
   if (C.reconstruction == 2) {
-    const T kappa = T(1.0 / 3.0);
-    const T w1 = T(0.25) * (T(1) - kappa), w2 = T(0.25) * (T(1) + kappa);
 #pragma unroll
     for (int l = 0; l < NV; ++l) {
       if (l < nv) {
@@ -350,9 +358,9 @@ __device__ __forceinline__ void face_inviscid(const ChemParams &C, const T *rec,
         const T d_i2 = v[3][l] - v[2][l];
         const T m1 = minmod(d_i, d_i1);
         const T m2 = minmod(d_i1, d_i2);
-        // minmod is symmetric: (1-k) mm(a,b) + (1+k) mm(b,a) = 2 mm(a,b)
-        L[l] = v[1][l] + (w1 * m1 + w2 * m1);
-        R[l] = v[2][l] - (w1 * m2 + w2 * m2);
+        // minmod is symmetric: ((1-k) mm(a,b) + (1+k) mm(b,a)) / 4 = mm(a,b) / 2
+        L[l] = v[1][l] + T(0.5) * m1;
+        R[l] = v[2][l] - T(0.5) * m2;
       }
     }
   } else {

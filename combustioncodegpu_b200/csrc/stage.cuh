@@ -16,7 +16,8 @@
 // [f * N + p], point p = BlockInfo.base + i + nx*j + nx*ny*k.
 //   P   : rho, u, v, w, p, T, Y_0..Y_{ns-1}         (bulk precision T)
 //   Pr  : mu, lambda, rhoD_0..rhoD_{ns-1}           (bulk precision T)
-//   G   : J, xi_x, xi_y, xi_z, eta_x, ..., zeta_z   (bulk precision T)
+//   G   : J and the metrics, FP32 per direction d (J, grad xi_d) as a group of
+//         four, [3][N][4], then J again, [N]; FP64 ten fields (geo_row, geo_jac)
 //   Q   : rho, rho u, rho v, rho w, rho E, rho Y_k  (FP64 always)
 #pragma once
 #include "physics.cuh"
@@ -26,6 +27,108 @@ namespace ccb {
 __device__ __forceinline__ void atomic_min_pos_double(unsigned long long *dst, double v) {
   if (!(v > 0.0) || !(v < 1e300)) return;
   atomicMin(dst, (unsigned long long)__double_as_longlong(v));
+}
+
+// Geometry of a point.  FP32: a face reads J and one metric row per direction
+// at both of its points, so these four values are one 16-byte load, and the
+// plain J serves the update, which needs nothing else of the geometry.  FP64:
+// ten fields, [10][N] (rows as two 16-byte loads: faces 0.366 -> 0.376 ms).
+template <typename T>
+struct GeoRow {
+  T J, m[3];
+};
+__device__ __forceinline__ GeoRow<float> geo_row(const float *__restrict__ G, int N, int d, int p) {
+  const float4 v = *reinterpret_cast<const float4 *>(G + 4 * (d * N + p));
+  return {v.x, {v.y, v.z, v.w}};
+}
+__device__ __forceinline__ GeoRow<double> geo_row(const double *__restrict__ G, int N, int d, int p) {
+  return {G[p], {G[(1 + 3 * d) * N + p], G[(2 + 3 * d) * N + p], G[(3 + 3 * d) * N + p]}};
+}
+__device__ __forceinline__ float geo_jac(const float *__restrict__ G, int N, int p) { return G[12 * N + p]; }
+__device__ __forceinline__ double geo_jac(const double *__restrict__ G, int, int p) { return G[p]; }
+
+// Face arena of the split variant, [3][group][N][width] with face_stride
+// values per direction and point.  FP32: the n_var fluxes of a face in groups
+// of four (16-byte accesses; a remainder of at most two is a group of two), so
+// that a face is written and read in a quarter of the instructions: 128^3, 9
+// species, faces 0.479 -> 0.440 ms per stage (with the geometry rows).  FP64:
+// one value per group; pairs cost the update more registers in flight than
+// they save instructions (97 x 85 x 71: update 0.249 -> 0.272 ms, faces equal).
+template <typename T>
+constexpr int kFaceGroup = sizeof(T) == 4 ? 4 : 1;
+template <typename T, int NV>
+constexpr int kFaceGroups = (NV + kFaceGroup<T> - 1) / kFaceGroup<T>;
+
+// Group g (variables W g.., W = kFaceGroup) of the faces at point p of one
+// direction, into x[0..W-1] (x[2], x[3] untouched where the group has two).
+__device__ __forceinline__ void load_faces(const float *__restrict__ Fd, int N, int nv, int g, int p, float *x) {
+  const float *base = Fd + 4 * g * N;
+  if (nv - 4 * g > 2) {
+    const float4 v = reinterpret_cast<const float4 *>(base)[p];
+    x[0] = v.x, x[1] = v.y, x[2] = v.z, x[3] = v.w;
+  } else {
+    const float2 v = reinterpret_cast<const float2 *>(base)[p];
+    x[0] = v.x, x[1] = v.y;
+  }
+}
+__device__ __forceinline__ void load_faces(const double *__restrict__ Fd, int N, int, int g, int p, double *x) {
+  x[0] = Fd[g * N + p];
+}
+
+__device__ __forceinline__ void store_group(float *__restrict__ Fd, int N, int nv, int g, int p, const float *x) {
+  float *base = Fd + 4 * g * N;
+  if (nv - 4 * g > 2)
+    reinterpret_cast<float4 *>(base)[p] = make_float4(x[0], x[1], x[2], x[3]);
+  else
+    reinterpret_cast<float2 *>(base)[p] = make_float2(x[0], x[1]);
+}
+__device__ __forceinline__ void store_group(double *__restrict__ Fd, int N, int, int g, int p, const double *x) {
+  Fd[g * N + p] = x[0];
+}
+
+// The residual's sum over the directions of F(+1/2) - F(-1/2) for the
+// variables of group g at point p (the fused kernel's order), with the
+// minus-side faces at px, py, pz; without a third direction pz = p, whose
+// difference is zero (the arena starts zeroed): a branch around the loads
+// would keep the compiler from batching them over the groups (97 x 85 x 71
+// FP64: update 0.25 against 0.29 ms per stage).
+template <typename T>
+__device__ __forceinline__ void face_sum(const T *__restrict__ Fx, const T *__restrict__ Fy, const T *__restrict__ Fz,
+                                         int N, int nv, int g, int p, int px, int py, int pz,
+                                         T (&acc)[kFaceGroup<T>]) {
+  constexpr int W = kFaceGroup<T>;
+  T x0[W], x1[W], y0[W], y1[W], z0[W], z1[W];
+  load_faces(Fx, N, nv, g, p, x1), load_faces(Fx, N, nv, g, px, x0);
+  load_faces(Fy, N, nv, g, p, y1), load_faces(Fy, N, nv, g, py, y0);
+  load_faces(Fz, N, nv, g, p, z1), load_faces(Fz, N, nv, g, pz, z0);
+#pragma unroll
+  for (int i = 0; i < W; ++i) {
+    if (W * g + i >= nv) continue;
+    acc[i] = x1[i] - x0[i];
+    acc[i] += y1[i] - y0[i];
+    acc[i] += z1[i] - z0[i];
+  }
+}
+
+// The fluxes F of face d of point p into the face arena.
+template <typename T, int NV>
+__device__ __forceinline__ void store_faces(T *__restrict__ faces, int N, int nv, int d, int p, const T (&F)[NV]) {
+  constexpr int W = kFaceGroup<T>;
+  if constexpr (W == 1) {
+#pragma unroll
+    for (int l = 0; l < NV; ++l)
+      if (l < nv) faces[(d * nv + l) * N + p] = F[l];
+    return;
+  }
+  T *Fd = faces + (int64_t)d * face_stride(nv, (int)sizeof(T)) * N;
+#pragma unroll
+  for (int g = 0; g < kFaceGroups<T, NV>; ++g) {
+    if (W * g >= nv) continue;
+    T x[W];
+#pragma unroll
+    for (int i = 0; i < W; ++i) x[i] = W * g + i < NV ? F[W * g + i < NV ? W * g + i : 0] : T(0);
+    store_group(Fd, N, nv, g, p, x);
+  }
 }
 
 // TemporalScheme.cu:11-43: CFL / (inviscid + viscous spectral radius), from
@@ -56,7 +159,11 @@ __device__ __forceinline__ double local_time_step(const ChemParams &C, const T *
                                                   bool three_d) {
   double m[9];
 #pragma unroll
-  for (int r = 0; r < 9; ++r) m[r] = (double)G[(1 + r) * N + p];
+  for (int d = 0; d < 3; ++d) {
+    const GeoRow<T> g = geo_row(G, (int)N, d, (int)p);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) m[3 * d + c] = (double)g.m[c];
+  }
   return local_time_step_m(C, m, rho, u, v, w, c, gamma, mu, three_d);
 }
 
@@ -114,9 +221,11 @@ __device__ __forceinline__ void face_flux_gen(const ChemParams &C, const T *rec,
       if (l < ns) v[t][5 + l] = S.at(6 + l, t - 1);
   }
   T k[3];
-  const T J0 = G[p], J1 = G[p1];
+  {
+    const GeoRow<T> g0 = geo_row(G, N, d, p), g1 = geo_row(G, N, d, p1);
 #pragma unroll
-  for (int c = 0; c < 3; ++c) k[c] = T(0.5) * (J0 * G[(1 + 3 * d + c) * N + p] + J1 * G[(1 + 3 * d + c) * N + p1]);
+    for (int c = 0; c < 3; ++c) k[c] = T(0.5) * (g0.J * g0.m[c] + g1.J * g1.m[c]);
+  }
   face_inviscid<T, NS>(C, rec, v, k, F);
   if (!C.viscous) return;
   // the face's transport properties first: their loads (through L1, from the
@@ -139,9 +248,10 @@ __device__ __forceinline__ void face_flux_gen(const ChemParams &C, const T *rec,
   for (int q = 0; q < 3; ++q) {
     const int r = q == 0 ? d : tangent(d, q);
     const T w = q == 0 ? T(0.5) : T(0.125);
+    const GeoRow<T> g0 = geo_row(G, N, r, p), g1 = geo_row(G, N, r, p1);
     T m[3], D3[3];
 #pragma unroll
-    for (int c = 0; c < 3; ++c) m[c] = w * (G[(1 + 3 * r + c) * N + p] + G[(1 + 3 * r + c) * N + p1]);
+    for (int c = 0; c < 3; ++c) m[c] = w * (g0.m[c] + g1.m[c]);
     a[q] = m[0] * k[0] + m[1] * k[1] + m[2] * k[2];
 #pragma unroll
     for (int c = 0; c < 3; ++c) D3[c] = S.diff(1 + c, q);
@@ -209,16 +319,28 @@ __device__ __forceinline__ void gamma_and_c(const ChemParams &C, const T *rec, T
 // the new state (Field.cu:178-210), |V| for the residual and the point's
 // contribution to the next global time step.
 // The conserved variable l of point p after the RK stage, from its residual
-// dq (TimeAdvanceFunc.cu:255-265; SSP-RK3 combination).
+// dql, the geometric term gcl of its direction (l = 1..3) and the states qin
+// and qn (TimeAdvanceFunc.cu:255-265; SSP-RK3 combination; qn counts when
+// a.a != 0).
+template <typename T>
+__device__ __forceinline__ double stage_value(const ChemParams &C, const StageArgs<T> &a, int l, double dql, double gcl,
+                                              double dtj, bool three_d, double qin, double qn) {
+  // momentum fluxes carry p - p_ref: add back -p_ref sum(k+ - k-) (zero on uniform grids)
+  if (a.gcl && l >= 1 && l <= 3) dql -= C.p_ref * gcl;
+  double qs = qin + dql * dtj;
+  if (l == 3 && !three_d) qs = 0;
+  double q = (a.a != 0.0) ? a.a * qn + a.b * qs : qs;
+  if (a.q32) q = (double)(float)q;  // full-FP32 study: FP32 conserved state
+  return q;
+}
 template <typename T>
 __device__ __forceinline__ double conserved_update(const ChemParams &C, const StageArgs<T> &a, int p, int N, int l,
                                                    double dql, double dtj, bool three_d) {
-  // momentum fluxes carry p - p_ref: add back -p_ref sum(k+ - k-) (zero on uniform grids)
   if (a.gcl && l >= 1 && l <= 3) dql -= C.p_ref * a.gcl[(l - 1) * N + p];
   double qs = a.Qin[l * N + p] + dql * dtj;
   if (l == 3 && !three_d) qs = 0;
   double q = (a.a != 0.0) ? a.a * a.Qn[l * N + p] + a.b * qs : qs;
-  if (a.q32) q = (double)(float)q;  // full-FP32 study: FP32 conserved state
+  if (a.q32) q = (double)(float)q;
   return q;
 }
 
@@ -342,8 +464,10 @@ __device__ __forceinline__ void point_finish(const ChemParams &C, const T *rec, 
 #pragma unroll
   for (int l = 0; l < A; ++l)
     if (l < ns) Prn[(2 + l) * N + p] = rd[l];
-  if (want_dt) {
-    const double dtl = local_time_step<T>(C, G, N, p, rho, u, v, w, (double)c, (double)gam, (double)mu, three_d);
+  if (want_dt) {  // density and velocity again from the state just stored, rather than kept in registers until here
+    const double rho_d = a.Qout[p], inv_d = 1.0 / rho_d;
+    const double dtl = local_time_step<T>(C, G, N, p, rho_d, a.Qout[N + p] * inv_d, a.Qout[2 * N + p] * inv_d,
+                                          a.Qout[3 * N + p] * inv_d, (double)c, (double)gam, (double)mu, three_d);
     dt_min = fmin(dt_min, dtl);
   }
 }
@@ -359,7 +483,7 @@ __device__ __forceinline__ void point_update(const ChemParams &C, const T *rec, 
   const int nv = 5 + ns;
   p = CCB_IDX(C, p, N);
   const T *__restrict__ G = a.G;
-  const double dtj = dt / (double)G[p];
+  const double dtj = dt / (double)geo_jac(G, N, p);
   // whether this point's step enters the next global time step, read with
   // the state rather than behind the stores below
   const bool want_dt = a.dt_next && !((a.skip_dt[p >> 5] >> (p & 31)) & 1u);
@@ -411,7 +535,18 @@ __device__ __forceinline__ void prefetch_planes(const StageArgs<T> &a, const Blo
     rows(a.P, np, k + 3, max(t.j0 - 2, -B.g), min(t.j0 + kTY + 2, B.my + B.g), i_lo, i_hi, e0);
   if (k + 2 <= kmax) {
     rows(a.Pr, npr, k + 2, max(t.j0 - 1, -B.g), min(t.j0 + kTY + 1, B.my + B.g), i_lo, i_hi, e0);
-    rows(a.G, 10, k + 2, max(t.j0 - 1, -B.g), min(t.j0 + kTY + 1, B.my + B.g), i_lo, i_hi, e0);
+    // geometry: ten fields, or (FP32, geo_row) three arrays of groups of four and the plain J
+    const int j_lo = max(t.j0 - 1, -B.g), j_hi = min(t.j0 + kTY + 1, B.my + B.g);
+    if (sizeof(T) == 8) {
+      rows(a.G, 10, k + 2, j_lo, j_hi, i_lo, i_hi, e0);
+    } else {
+      rows(a.G + 12 * (size_t)N, 1, k + 2, j_lo, j_hi, i_lo, i_hi, e0);
+      const int nr = j_hi - j_lo;
+      for (int e = tid; e < 3 * nr; e += kTX * kTY) {
+        const int row = (int)B.base + sk * (k + 2) + sj * (j_lo + e % nr);
+        l2_prefetch(a.G + (size_t)4 * (e / nr) * N, 4 * N, 4 * (row + i_lo), 4 * (row + i_hi));
+      }
+    }
   }
   if (k + 1 < t.k1) {
     rows(a.Qin, nv, k + 1, t.j0, min(t.j0 + kTY, B.my), t.i0, t.i0 + kTX, e0);
@@ -986,9 +1121,10 @@ __global__ void k_gcl(const BlockInfo *blocks, int nblocks, const T *G, int64_t 
     for (int d = 0; d < (B.mz > 1 ? 3 : 2); ++d) {
       const int64_t q0 = p - st[d], q1 = p, q2 = p + st[d];
       for (int c = 0; c < 3; ++c) {
-        const T *m = G + (1 + 3 * d + c) * N;
-        const T kp = T(0.5) * (G[q1] * m[q1] + G[q2] * m[q2]);
-        const T km = T(0.5) * (G[q0] * m[q0] + G[q1] * m[q1]);
+        const GeoRow<T> g0 = geo_row(G, (int)N, d, (int)q0), g1 = geo_row(G, (int)N, d, (int)q1),
+                        g2 = geo_row(G, (int)N, d, (int)q2);
+        const T kp = T(0.5) * (g1.J * g1.m[c] + g2.J * g2.m[c]);
+        const T km = T(0.5) * (g0.J * g0.m[c] + g1.J * g1.m[c]);
         acc[c] += (double)kp - (double)km;
       }
     }
@@ -996,7 +1132,25 @@ __global__ void k_gcl(const BlockInfo *blocks, int nblocks, const T *G, int64_t 
   }
 }
 
-// Global time step of the current state over interior points.// Global time step of the current state over interior points.
+// Geometry from the caller's fields J, m11, m12, .., m33 ([10][N], FP64).
+template <typename T>
+__global__ void k_geometry(const double *__restrict__ src, T *__restrict__ G, int64_t N) {
+  const int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (p >= N) return;
+  if constexpr (sizeof(T) == 8) {
+    for (int f = 0; f < 10; ++f) G[f * N + p] = src[f * N + p];
+  } else {
+    const T J = T(src[p]);
+    for (int d = 0; d < 3; ++d) {
+      T *row = G + 4 * (d * N + p);
+      row[0] = J;
+      for (int c = 0; c < 3; ++c) row[1 + c] = T(src[(1 + 3 * d + c) * N + p]);
+    }
+    G[12 * N + p] = J;
+  }
+}
+
+// Global time step of the current state over interior points.
 template <typename T, int NS>
 __global__ void k_dt_reduce(const __grid_constant__ ChemParams C, const BlockInfo *blocks, int nblocks, const T *P,
                             const T *Pr, const T *G, int64_t N, int64_t n_interior_total,

@@ -1,7 +1,7 @@
 // Split stage: faces first, then the point update (sm_100a).
 //
 // k_faces computes every face flux of the stage exactly once and writes it
-// to the face arena; k_update differences the six faces of each point and
+// to the face arena (grouped, store_faces); k_update differences the six faces of each point and
 // applies the same RK update, FP64 Newton, transport and time-step reduction
 // as the fused kernel (point_update).  Splitting costs one write and one read
 // of the face fluxes (3 n_var values per point) but removes the fused
@@ -41,11 +41,7 @@ __global__ void __launch_bounds__(kTX *kTY, sizeof(T) == 8 ? 1 : 2)
   const int N = (int)a.N, sj = B.nx, sk = B.nx * B.ny;
   const bool three_d = B.mz > 1;
   T F[NV];
-  auto put = [&](int d, int p) {
-#pragma unroll
-    for (int l = 0; l < NV; ++l)
-      if (l < nv) a.faces[(d * nv + l) * N + p] = F[l];
-  };
+  auto put = [&](int d, int p) { store_faces<T, NV>(a.faces, N, nv, d, p, F); };
   if (!edge) {
     const int i = t.i0 + tx, j = t.j0 + ty;
     if (i >= B.mx || j >= B.my) return;
@@ -111,8 +107,8 @@ __global__ void __launch_bounds__(256, MINB)
   const bool three_d = B.mz > 1;
   const T *__restrict__ P = a.P;
   const T *__restrict__ Fx = a.faces;
-  const T *__restrict__ Fy = a.faces + (size_t)nv * N;
-  const T *__restrict__ Fz = a.faces + (size_t)2 * nv * N;
+  const T *__restrict__ Fy = a.faces + (size_t)face_stride(nv, (int)sizeof(T)) * N;
+  const T *__restrict__ Fz = a.faces + (size_t)2 * face_stride(nv, (int)sizeof(T)) * N;
   unsigned flags = 0;
   double dt_min = 1e300;
   if (act) {
@@ -135,7 +131,7 @@ __global__ void __launch_bounds__(256, MINB)
       } else {
         dt = dt_global;
       }
-      const double dtj = dt / (double)a.G[p];
+      const double dtj = dt / (double)geo_jac(a.G, N, p);
       // whether this point's step enters the next global time step, read with
       // the state rather than behind the stores
       const bool want_dt = a.dt_next && !((a.skip_dt[p >> 5] >> (p & 31)) & 1u);
@@ -149,15 +145,17 @@ __global__ void __launch_bounds__(256, MINB)
           if (l < nv) q[l] = conserved_update<T>(C, a, p, N, l, (double)Fx[l * N + p], dtj, three_d);
       } else {
         // the minus-side faces (checked in bounds-checked builds)
-        const int px = CCB_IDX(C, p - 1, N), py = CCB_IDX(C, p - sj, N), pz = CCB_IDX(C, p - sk, N);
+        const int px = CCB_IDX(C, p - 1, N), py = CCB_IDX(C, p - sj, N), pz = CCB_IDX(C, three_d ? p - sk : p, N);
+        constexpr int W = kFaceGroup<T>;
 #pragma unroll
-        for (int l = 0; l < NV; ++l) {
-          if (l < nv) {
-            const int o = l * N + p;
-            T acc = Fx[o] - Fx[l * N + px];
-            acc += Fy[o] - Fy[l * N + py];
-            if (three_d) acc += Fz[o] - Fz[l * N + pz];
-            q[l] = conserved_update<T>(C, a, p, N, l, -(double)acc, dtj, three_d);
+        for (int g = 0; g < kFaceGroups<T, NV>; ++g) {
+          if (W * g >= nv) continue;
+          T acc[W];
+          face_sum<T>(Fx, Fy, Fz, N, nv, g, p, px, py, pz, acc);
+#pragma unroll
+          for (int i = 0; i < W; ++i) {
+            const int l = W * g + i;
+            if (l < NV && l < nv) q[l < NV ? l : 0] = conserved_update<T>(C, a, p, N, l, -(double)acc[i], dtj, three_d);
           }
         }
       }

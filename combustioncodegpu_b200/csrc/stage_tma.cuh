@@ -377,7 +377,7 @@ __device__ __forceinline__ void prefetch_props_geometry(const StageArgs<T> &a, c
   const int N = (int)a.N, sj = B.nx, sk = B.nx * B.ny;
   const int j_lo = max(t.j0 - 1, -B.g), j_hi = min(t.j0 + TY + 1, B.my + B.g), nr = j_hi - j_lo;
   const int n = (npr + 10) * nr;
-  for (int e = tid; e < n; e += TX * TY) {
+  for (int e = tid; e < n; e += TX * TY) {  // FP64: ten geometry fields (geo_row)
     const int f = e / nr, j = j_lo + e % nr;
     const T *base = f < npr ? a.Pr + (size_t)f * N : a.G + (size_t)(f - npr) * N;
     const int row = (int)B.base + sk * kp + sj * j;
@@ -460,9 +460,7 @@ __device__ __forceinline__ int faces_tma_tile(const StageArgs<T> &a, const CUten
         const int sd = d == 0 ? 1 : (d == 1 ? sj : sk);
         const SmemStencilT<T, L::HX, L::PV> S(plm, pl0, pl1, pl2, q, d);
         face_flux_gen<T, NS>(C, sRec, S, a.Pr, a.G, N, p, sd, d, F);
-#pragma unroll
-        for (int l = 0; l < NV; ++l)
-          if (l < nv) a.faces[(d * nv + l) * N + p] = F[l];
+        store_faces<T, NV>(a.faces, N, nv, d, p, F);
       }
     }
     __syncthreads();  // plane k-1 is no longer read
