@@ -177,10 +177,12 @@ struct GridBarrier {
 
 // Node levels the single-launch halo program takes (more fall back to one
 // launch per level), and their bounds in the node list.
-constexpr int kHaloMaxLevels = 8;
+constexpr int kHaloMaxLevels = 32;
+constexpr int kHaloTailNodes = 128;  // a tail level (run by one CTA, one node a thread) has at most this many nodes
 struct HaloLevels {
   int64_t begin[kHaloMaxLevels + 1];
   int n;
+  int n_grid;  // leading levels run by the whole grid; the others by one CTA
 };
 
 // Arguments of one stage launch (see stage.cuh).

@@ -93,13 +93,15 @@ CCB_DECLARE_COUNTS(float)
 #undef CCB_DECLARE
 
 // Non-templated helpers (misc.cu).
-// dst = (float)(src - shift), dst = (double)src + shift (the gauge pressure field)
+// dst = (float)(src - shift) (the gauge pressure field)
 cudaError_t launch_convert_d2f_shift(const double *src, float *dst, int64_t n, double shift, cudaStream_t s);
-cudaError_t launch_convert_f2d_shift(const float *src, double *dst, int64_t n, double shift, cudaStream_t s);
 cudaError_t launch_convert_d2f(const double *src, float *dst, int64_t n, cudaStream_t s);
-cudaError_t launch_convert_f2d(const float *src, double *dst, int64_t n, cudaStream_t s);
 cudaError_t launch_dt_finalize(double *dt, unsigned long long *dt_next, unsigned *status, double *dt_hist,
                                cudaStream_t s);
+// nf fields of a block's ghosted box, packed [nf][Ng] FP64; shift is added to field shift_f (-1: none)
+template <typename T>
+cudaError_t launch_pack_box(const T *src, int64_t N, const BlockInfo &B, int nf, int shift_f, double shift, double *out,
+                            cudaStream_t s);
 cudaError_t launch_zero_points(double *field, const int64_t *points, int64_t n, cudaStream_t s);
 template <typename T>
 cudaError_t launch_gather_points(const T *src, int64_t N, int nf, const int64_t *idx, int64_t n, double *out,

@@ -12,20 +12,9 @@ __global__ void k_convert_d2f(const double *src, float *dst, int64_t n) {
   if (i < n) dst[i] = (float)src[i];
 }
 
-__global__ void k_convert_f2d(const float *src, double *dst, int64_t n) {
-  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i < n) dst[i] = (double)src[i];
-}
-
 cudaError_t launch_convert_d2f(const double *src, float *dst, int64_t n, cudaStream_t s) {
   if (n <= 0) return cudaSuccess;
   k_convert_d2f<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(src, dst, n);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_convert_f2d(const float *src, double *dst, int64_t n, cudaStream_t s) {
-  if (n <= 0) return cudaSuccess;
-  k_convert_f2d<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(src, dst, n);
   return cudaGetLastError();
 }
 
@@ -34,22 +23,40 @@ __global__ void k_convert_d2f_shift(const double *src, float *dst, int64_t n, do
   if (i < n) dst[i] = (float)(src[i] - shift);
 }
 
-__global__ void k_convert_f2d_shift(const float *src, double *dst, int64_t n, double shift) {
-  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i < n) dst[i] = (double)src[i] + shift;
-}
-
 cudaError_t launch_convert_d2f_shift(const double *src, float *dst, int64_t n, double shift, cudaStream_t s) {
   if (n <= 0) return cudaSuccess;
   k_convert_d2f_shift<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(src, dst, n, shift);
   return cudaGetLastError();
 }
 
-cudaError_t launch_convert_f2d_shift(const float *src, double *dst, int64_t n, double shift, cudaStream_t s) {
-  if (n <= 0) return cudaSuccess;
-  k_convert_f2d_shift<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(src, dst, n, shift);
+// Fields of one block's ghosted box, packed as the host takes them:
+// out[f][(mx + 2g)(my + 2g)(mz + 2g)] in FP64 from arena fields of row pitch
+// nx, field shift_f raised by shift (the gauge pressure).
+template <typename T>
+__global__ void k_pack_box(const T *__restrict__ src, int64_t N, int64_t off, int nx, int ny, int wx, int wy, int64_t ng,
+                           int shift_f, double shift, double *__restrict__ out) {
+  const int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (e >= ng) return;
+  const int f = blockIdx.y;
+  const int r = (int)(e / wx), i = (int)(e % wx), j = r % wy, k = r / wy;
+  const double v = (double)src[f * N + off + i + (int64_t)nx * (j + (int64_t)ny * k)];
+  out[f * ng + e] = f == shift_f ? v + shift : v;
+}
+
+template <typename T>
+cudaError_t launch_pack_box(const T *src, int64_t N, const BlockInfo &B, int nf, int shift_f, double shift, double *out,
+                            cudaStream_t s) {
+  const int wx = B.mx + 2 * B.g, wy = B.my + 2 * B.g;
+  const int64_t ng = (int64_t)wx * wy * (B.mz + 2 * B.g);
+  if (ng <= 0 || nf <= 0) return cudaSuccess;
+  k_pack_box<T><<<dim3((unsigned)((ng + 255) / 256), nf), 256, 0, s>>>(src, N, B.off, B.nx, B.ny, wx, wy, ng, shift_f,
+                                                                      shift, out);
   return cudaGetLastError();
 }
+template cudaError_t launch_pack_box<float>(const float *, int64_t, const BlockInfo &, int, int, double, double *,
+                                            cudaStream_t);
+template cudaError_t launch_pack_box<double>(const double *, int64_t, const BlockInfo &, int, int, double, double *,
+                                             cudaStream_t);
 
 // dt <- dt_next (when a candidate was reduced), dt_next <- +inf; the step's
 // dt is appended to the history slot.

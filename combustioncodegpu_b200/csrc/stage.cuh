@@ -794,7 +794,8 @@ __device__ __forceinline__ void halo_node(const HaloArgs<T> &a, const ChemParams
     for (int f = 0; f < 6 + A; ++f)
       if (f < 6 + ns) {
         same = same && (xa[f] == xb[f]);
-        a.sP[f * S + o] = T(0.5) * (xb[f] + xa[f]);
+        xa[f] = T(0.5) * (xb[f] + xa[f]);
+        a.sP[f * S + o] = xa[f];
       }
 #pragma unroll
     for (int f = 0; f < 5 + A; ++f)
@@ -806,10 +807,11 @@ __device__ __forceinline__ void halo_node(const HaloArgs<T> &a, const ChemParams
       return;
     }
     // averaged state: recompute its transport properties below
-    for (int f = 0; f < 6; ++f) pr[f] = (double)a.sP[f * S + o];
+#pragma unroll
+    for (int f = 0; f < 6; ++f) pr[f] = (double)xa[f];
 #pragma unroll
     for (int l = 0; l < A; ++l)
-      if (l < ns) Y[l] = (double)a.sP[(6 + l) * S + o];
+      if (l < ns) Y[l] = (double)xa[6 + l];
   } else {
     const BcDevice &bc = a.bcs[nd.bc];
     if (nd.op == kHaloInflow) {
@@ -1038,7 +1040,11 @@ __device__ __forceinline__ bool grid_sync_bounded(GridBarrier *bar, long long ma
 // Phase A in one cooperative launch: the node levels with a grid-wide
 // barrier between levels (every node of a level reads only the state and
 // lower levels).  A barrier that gives up sets kStatusHaloTimeout and the
-// CTA returns.
+// CTA returns.  From level lv.n_grid on every level is small (corners of
+// corners: at most kHaloTailNodes nodes) and CTA 0 runs them alone, with its
+// own barrier between levels: twelve uneven blocks have 18 levels, of which
+// the last eight hold less than a CTA's worth of nodes each and cost a launch
+// or a grid barrier more than their work.
 template <typename T, int NS>
 __global__ void __launch_bounds__(128)
     k_halo_levels(const HaloArgs<T> a, const __grid_constant__ ChemParams C, const HaloLevels lv, GridBarrier *bar,
@@ -1046,11 +1052,16 @@ __global__ void __launch_bounds__(128)
   const int64_t tid = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int l = 0; l < lv.n; ++l) {
-    if (l > 0 && !grid_sync_bounded(bar, C.max_spins)) {
+    const bool tail = l >= lv.n_grid;
+    if (l > lv.n_grid) {
+      __syncthreads();  // this level reads slots that this CTA wrote
+    } else if (l > 0 && !grid_sync_bounded(bar, C.max_spins)) {
       if (threadIdx.x == 0) atomicOr(status, kStatusHaloTimeout);
       return;
     }
-    for (int64_t e = lv.begin[l] + tid; e < lv.begin[l + 1]; e += stride) halo_node<T, NS>(a, C, e);
+    if (tail && blockIdx.x != 0) return;
+    for (int64_t e = lv.begin[l] + (tail ? threadIdx.x : tid); e < lv.begin[l + 1]; e += stride)
+      halo_node<T, NS>(a, C, e);
   }
 }
 
