@@ -212,10 +212,9 @@ struct StageArgs {
   const double *gcl;         // [3][N]: sum over directions of k(+) - k(-) per point (p_ref != 0), else null
   // split variant (stage_split.cuh): face fluxes (store_faces; face d of
   // point p lies between p and p + e_d), the tiles of the minus-side face
-  // layers (i, j or k = -1; direction in Tile::pad0), regular tile count
+  // layers (i, j or k = -1; direction in Tile::pad0)
   T *faces;
   const Tile *edge_tiles;
-  int n_regular;
   // 1: `faces` holds the residual dq [n_var][N] of every interior point
   // (k_faces_dq), which k_update reads as it is instead of differencing faces
   int dq_direct;

@@ -37,10 +37,9 @@ size_t Launch<T, NS>::update_smem() {
 template <typename T, int NS>
 cudaError_t Launch<T, NS>::faces(const StageArgs<T> &a, const ChemParams &C, int n_regular, int n_edge,
                                  cudaStream_t s) {
-  if (n_regular + n_edge <= 0) return cudaSuccess;
-  StageArgs<T> b = a;
-  b.n_regular = n_regular;
-  k_faces<T, NS><<<n_regular + n_edge, dim3(kTX, kTY), faces_smem(), s>>>(b, C);
+  if (n_regular > 0) k_faces<T, NS><<<n_regular, dim3(kTX, kTY), faces_smem(), s>>>(a, C);
+  if (n_edge > 0)
+    k_edge_faces<T, NS><<<n_edge * (kTY / kEdgeRows), dim3(kTX, kEdgeRows), faces_smem(), s>>>(a, C);
   return cudaGetLastError();
 }
 

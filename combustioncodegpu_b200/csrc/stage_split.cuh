@@ -35,29 +35,48 @@ __global__ void __launch_bounds__(kTX *kTY, sizeof(T) == 8 ? 1 : 2)
   for (int e = tid, nrec = ns * kRecRanges * kRecLen; e < nrec; e += kTX * kTY) sRec[e] = param_rec<T>(C)[e];
   __syncthreads();  // the only barrier: threads may leave from here on
 
-  const bool edge = (int)blockIdx.x >= a.n_regular;
-  const Tile t = edge ? a.edge_tiles[blockIdx.x - a.n_regular] : a.tiles[blockIdx.x];
+  const Tile t = a.tiles[blockIdx.x];
   const BlockInfo B = a.blocks[t.blk];
   const int N = (int)a.N, sj = B.nx, sk = B.nx * B.ny;
   const bool three_d = B.mz > 1;
   T F[NV];
-  auto put = [&](int d, int p) { store_faces<T, NV>(a.faces, N, nv, d, p, F); };
-  if (!edge) {
-    const int i = t.i0 + tx, j = t.j0 + ty;
-    if (i >= B.mx || j >= B.my) return;
-    const int col = (int)B.base + i + sj * j;
-    for (int k = t.k0; k < t.k1; ++k) {
-      const int p = col + sk * k;
+  const int i = t.i0 + tx, j = t.j0 + ty;
+  if (i >= B.mx || j >= B.my) return;
+  const int col = (int)B.base + i + sj * j;
+  for (int k = t.k0; k < t.k1; ++k) {
+    const int p = col + sk * k;
 #pragma unroll 1
-      for (int it = three_d ? 0 : 1; it < 3; ++it) {
-        const int d = it == 0 ? 2 : it - 1;
-        const int sd = d == 0 ? 1 : (d == 1 ? sj : sk);
-        face_flux<T, NS>(C, sRec, a.P, a.Pr, a.G, N, p, d, sd, sj, sk, F);
-        put(d, p);
-      }
+    for (int it = three_d ? 0 : 1; it < 3; ++it) {
+      const int d = it == 0 ? 2 : it - 1;
+      const int sd = d == 0 ? 1 : (d == 1 ? sj : sk);
+      face_flux<T, NS>(C, sRec, a.P, a.Pr, a.G, N, p, d, sd, sj, sk, F);
+      store_faces<T, NV>(a.faces, N, nv, d, p, F);
     }
-    return;
   }
+}
+
+// The edge tiles: one face per thread, kEdgeRows rows of a tile per CTA.
+// There are few faces here and each is a long chain of loads (at i = -1 one
+// sector per lane), so the launch takes as long as its busiest SM: CTAs of two
+// warps spread them over all SMs, where CTAs of a whole tile (eight warps)
+// filled some of them and left the others idle: 97 x 85 x 71 FP64 faces 0.363
+// -> 0.348 ms a stage, 113 x 66 x 33 mixed 0.113 -> 0.087 ms, 128^3 43 -> 38 us.
+constexpr int kEdgeRows = 2;
+template <typename T, int NS>
+__global__ void __launch_bounds__(kTX *kEdgeRows, sizeof(T) == 8 ? 4 : 8)
+    k_edge_faces(const StageArgs<T> a, const __grid_constant__ ChemParams C) {
+  constexpr int NV = 5 + SpecCount<NS>::kArr;
+  const int ns = SpecCount<NS>::n(C);
+  const int nv = 5 + ns;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  T *sRec = reinterpret_cast<T *>(smem_raw);  // [A][kRecRanges][kRecLen]
+  const int tx = threadIdx.x, tid = threadIdx.y * kTX + tx;
+  const Tile t = a.edge_tiles[blockIdx.x / (kTY / kEdgeRows)];
+  const int ty = (int)(blockIdx.x % (kTY / kEdgeRows)) * kEdgeRows + threadIdx.y;  // row of the tile
+  const BlockInfo B = a.blocks[t.blk];
+  for (int e = tid, nrec = ns * kRecRanges * kRecLen; e < nrec; e += kTX * kEdgeRows) sRec[e] = param_rec<T>(C)[e];
+  __syncthreads();
+  const int N = (int)a.N, sj = B.nx, sk = B.nx * B.ny;
   const int d = t.pad0;
   int i, j, k;
   bool ok;
@@ -69,13 +88,14 @@ __global__ void __launch_bounds__(kTX *kTY, sizeof(T) == 8 ? 1 : 2)
     ok = i < B.mx && k < t.k1;
   } else {
     i = t.i0 + tx, j = t.j0 + ty, k = -1;
-    ok = i < B.mx && j < B.my && three_d;
+    ok = i < B.mx && j < B.my && B.mz > 1;
   }
   if (!ok) return;
   const int p = (int)B.base + i + sj * j + sk * k;
   const int sd = d == 0 ? 1 : (d == 1 ? sj : sk);
+  T F[NV];
   face_flux<T, NS>(C, sRec, a.P, a.Pr, a.G, N, p, d, sd, sj, sk, F);
-  put(d, p);
+  store_faces<T, NV>(a.faces, N, nv, d, p, F);
 }
 
 // MINB: CTAs per SM the registers are sized for (the autotuner tries 4 in
