@@ -1247,17 +1247,32 @@ int autotune(cc_ctx *c) {
     if (v.empty() && (variant < 3 || variant > 4)) v.push_back(32);
     return v;
   };
-  // three launches of one candidate after one untimed: ms each
-  auto timed = [&](auto &&launch, double &ms) -> int {
-    if (int r = launch()) return r;
+  // n launches of one candidate: ms each
+  auto batch = [&](auto &&launch, int n, double &ms) -> int {
     CK(cudaEventRecord(e0, c->stream));
-    for (int i = 0; i < 3; ++i)
+    for (int i = 0; i < n; ++i)
       if (int r = launch()) return r;
     CK(cudaEventRecord(e1, c->stream));
     CK(cudaEventSynchronize(e1));
     float t = 0;
     CK(cudaEventElapsedTime(&t, e0, e1));
-    ms = t / 3;
+    ms = t / n;
+    return 0;
+  };
+  // the better of two batches after an untimed launch; before the first
+  // candidate the GPU is kept busy for 10 ms (an idle GPU's first launches are
+  // slow, which made the early candidates lose now and then: 128^3 steps of
+  // 2.55 or 2.9 ms)
+  bool warm = false;
+  auto timed = [&](auto &&launch, double &ms) -> int {
+    double t = 0, busy = 0;
+    for (int n = 0; !warm && busy < 10.0 && n < 2000; ++n, busy += t)
+      if (int r = batch(launch, 1, t)) return r;
+    warm = true;
+    if (int r = launch()) return r;
+    if (int r = batch(launch, 2, ms)) return r;
+    if (int r = batch(launch, 2, t)) return r;
+    ms = std::min(ms, t);
     return 0;
   };
   auto set_tiles = [&](int kz, int ty, int tx) -> int {
