@@ -791,8 +791,8 @@ HaloArgs<T> halo_args(cc_ctx *c, int pn, int pp, double *qn, const double *qp) {
 
 // The halo program after a stage: the node levels (one cooperative launch
 // with a grid barrier between levels, or, in the per-block launch mode of the
-// reference's granularity and for programs of more than kHaloMaxLevels
-// levels, one launch per level), then one launch for the copies, the
+// reference's granularity and for programs of many wide levels, one launch
+// per level), then one launch for the copies, the
 // post-exchange time step and the zeroing of |V| at wall faces (vel).  Both
 // forms run the same device functions: identical results.
 template <typename T, int NS>
@@ -803,7 +803,14 @@ int run_halo(cc_ctx *c, int pn, int pp, double *qn, const double *qp, unsigned l
   h.dt_next = dt_next;
   const auto &lb = c->plan.level_begin;
   const int n_levels = lb.empty() ? 0 : (int)lb.size() - 1;
-  if (n_levels > 0 && !c->per_block && c->halo_coop && n_levels <= kHaloMaxLevels) {
+  // Beyond kHaloFewLevels levels the grid barriers (one per large level) pay
+  // against launches while the widest level is about one wave of CTAs (112 k
+  // nodes, 18 levels: 0.302 against 0.308 ms); on 64 blocks (682 k nodes, 18
+  // levels) one cooperative launch took 1.67 ms, launches 1.61.
+  int64_t widest = 0;
+  for (int l = 0; l < n_levels; ++l) widest = std::max(widest, lb[l + 1] - lb[l]);
+  const bool one_launch = n_levels <= kHaloFewLevels || (n_levels <= kHaloMaxLevels && widest <= kHaloWideNodes);
+  if (n_levels > 0 && !c->per_block && c->halo_coop && one_launch) {
     HaloLevels lv{};
     lv.n = n_levels;
     for (int l = 0; l <= n_levels; ++l) lv.begin[l] = lb[l];

@@ -178,6 +178,8 @@ struct GridBarrier {
 // Node levels the single-launch halo program takes (more fall back to one
 // launch per level), and their bounds in the node list.
 constexpr int kHaloMaxLevels = 32;
+constexpr int kHaloFewLevels = 8;        // always in one launch
+constexpr int64_t kHaloWideNodes = 1 << 18;  // more levels than that: while no level has more nodes
 constexpr int kHaloTailNodes = 128;  // a tail level (run by one CTA, one node a thread) has at most this many nodes
 struct HaloLevels {
   int64_t begin[kHaloMaxLevels + 1];
