@@ -803,10 +803,13 @@ int run_halo(cc_ctx *c, int pn, int pp, double *qn, const double *qp, unsigned l
   h.dt_next = dt_next;
   const auto &lb = c->plan.level_begin;
   const int n_levels = lb.empty() ? 0 : (int)lb.size() - 1;
-  // Beyond kHaloFewLevels levels the grid barriers (one per large level) pay
-  // against launches while the widest level is about one wave of CTAs (112 k
-  // nodes, 18 levels: 0.302 against 0.308 ms); on 64 blocks (682 k nodes, 18
-  // levels) one cooperative launch took 1.67 ms, launches 1.61.
+  // A program of more than kHaloFewLevels levels takes one launch only while no
+  // level has more than kHaloWideNodes nodes.  64 blocks (18 levels, 682 k nodes
+  // in the widest), per stage: one cooperative launch 1.63 ms, a launch per
+  // level 1.60, both builds measured in turn.  12 blocks (18 levels, 112 k
+  // averaged points): 0.302 ms in one launch; a launch per level took 0.307
+  // before the tail levels shared a CTA.  The line lies between these two
+  // programs; sizes between them were not measured.
   int64_t widest = 0;
   for (int l = 0; l < n_levels; ++l) widest = std::max(widest, lb[l + 1] - lb[l]);
   const bool one_launch = n_levels <= kHaloFewLevels || (n_levels <= kHaloMaxLevels && widest <= kHaloWideNodes);

@@ -175,8 +175,9 @@ struct GridBarrier {
   unsigned gen;
 };
 
-// Node levels the single-launch halo program takes (more fall back to one
-// launch per level), and their bounds in the node list.
+// Node levels the single-launch halo program takes (more, or more than
+// kHaloFewLevels with a wide one, run one launch per level), and their bounds
+// in the node list.
 constexpr int kHaloMaxLevels = 32;
 constexpr int kHaloFewLevels = 8;        // always in one launch
 constexpr int64_t kHaloWideNodes = 1 << 18;  // more levels than that: while no level has more nodes
