@@ -215,7 +215,7 @@ def issue_roofline(instr_per_point, npts, kernel_ms, sm_mhz):
     n_sm = torch.cuda.get_device_properties(0).multi_processor_count
     peak = n_sm * 4 * 32 * sm_mhz * 1e6  # thread instructions per second
     bound_ms = instr_per_point * npts / peak * 1e3
-    return {"thread_instructions_per_point": instr_per_point, "source": "ncu instruction mix (96^3 capture)",
+    return {"thread_instructions_per_point": instr_per_point, "source": "ncu instruction count (128^3 capture)",
             "issue_bound_ms": bound_ms, "kernel_ms": kernel_ms, "frac": bound_ms / kernel_ms,
             "peak": "%d SMs x 4 schedulers x 32 lanes x %.0f MHz" % (n_sm, sm_mhz)}
 
