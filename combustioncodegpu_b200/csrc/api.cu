@@ -601,7 +601,7 @@ int setup_device(cc_ctx *c) {
   int64_t n_int = 0;
   c->N = layout_blocks(c->blocks, c->ngg, c->hblocks, n_int);
   c->n_int = n_int;
-  if ((double)c->N * (6 + kMaxSpec) >= 2147483647.0)
+  if (!arena_fits(c->N))
     return fail(CC_ERR_ARG, "grid too large for one context (32-bit field offsets); split it over contexts");
 
   std::vector<HostBc> bcs = c->bcs;

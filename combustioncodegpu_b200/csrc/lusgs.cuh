@@ -106,8 +106,8 @@ __global__ void __launch_bounds__(kTX *kTY, sizeof(T) == 8 ? 1 : 2) k_lusgs_rhs(
   const T *__restrict__ P = a.P;
   const T *__restrict__ G = a.G;
   const T *__restrict__ Fx = a.faces;
-  const T *__restrict__ Fy = a.faces + (size_t)face_stride(nv, (int)sizeof(T)) * N;
-  const T *__restrict__ Fz = a.faces + (size_t)2 * face_stride(nv, (int)sizeof(T)) * N;
+  const T *__restrict__ Fy = a.faces + face_base(1, nv, (int)sizeof(T), N);
+  const T *__restrict__ Fz = a.faces + face_base(2, nv, (int)sizeof(T), N);
   // the residual of the variables of face group g at point p
   constexpr int W = kFaceGroup<T>;
   auto residual_group = [&](int p, int g, double (&dq)[W]) {

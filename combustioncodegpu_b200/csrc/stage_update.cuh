@@ -89,8 +89,8 @@ __global__ void __launch_bounds__(256, 2)
   const bool three_d = B.mz > 1;
   const T *__restrict__ P = a.P;
   const T *__restrict__ Fx = a.faces;
-  const T *__restrict__ Fy = a.faces + (size_t)face_stride(nv, (int)sizeof(T)) * N;
-  const T *__restrict__ Fz = a.faces + (size_t)2 * face_stride(nv, (int)sizeof(T)) * N;
+  const T *__restrict__ Fy = a.faces + face_base(1, nv, (int)sizeof(T), N);
+  const T *__restrict__ Fz = a.faces + face_base(2, nv, (int)sizeof(T), N);
   unsigned flags = 0, phase = 0;
   double dt_min = 1e300;
   const int col = (int)B.base + (act ? i + sj * j : 0);
