@@ -1230,9 +1230,10 @@ int autotune(cc_ctx *c) {
   }
   // tile heights of the TMA face kernels (variants 3-5; the other variants'
   // tiles are 32 x 8), those whose plane ring fits in shared memory
+  // (a pinned height of 16 is for FP32; FP64 takes it with 0 or 9 species only)
   std::vector<int> tys;
   for (int ty : {4, 8, 16})
-    if ((c->force_ty <= 0 || ty == c->force_ty) &&
+    if ((c->force_ty <= 0 || (ty == c->force_ty && (ty < 16 || c->precision != CC_FP64 || c->ns_key >= 0))) &&
         (Launch<T, NS>::faces_tma_smem(ty, 32) != 0 || Launch<T, NS>::faces_tma_smem(ty, 16) != 0))
       tys.push_back(ty);
   if (tys.empty()) return fail(CC_ERR_ARG, "the face tile height does not fit in shared memory in this precision");
