@@ -49,8 +49,22 @@ __device__ __forceinline__ double frcp(double a) { return 1.0 / a; }
 __device__ __forceinline__ float frcp(float a) { return __fdividef(1.0f, a); }
 __device__ __forceinline__ double fsqrt(double a) { return sqrt(a); }
 __device__ __forceinline__ float fsqrt(float a) { return a * rsqrtf(a); }
-__device__ __forceinline__ double frsqrt(double a) { return rsqrt(a); }
-__device__ __forceinline__ float frsqrt(float a) { return rsqrtf(a); }
+
+// Length of the face vector, from its square, and the reciprocal of that
+// length.  The mass flux takes the product of both, so what counts is that
+// they are reciprocal.  FP32: the reciprocal of the length as computed; the
+// reciprocal root itself leaves twice its error in the product, the same at
+// every face of a uniform grid (velocity error after 20 steps of the 32^3 box
+// 1.73e-7 against 1.30e-7).  FP64: its error is far below the rounding of the
+// fluxes, and root and division cost 1 % of the faces.
+__device__ __forceinline__ void length_and_reciprocal(double kk, double &len, double &inv) {
+  inv = rsqrt(kk);
+  len = kk * inv;
+}
+__device__ __forceinline__ void length_and_reciprocal(float kk, float &len, float &inv) {
+  len = fsqrt(kk);
+  inv = frcp(len);
+}
 
 // NASA-7 records (SpecTables::rec) are read through a pointer `rec` to the
 // [kMaxSpec][kRecRanges][kRecLen] array: the stage kernels point it at a copy
@@ -405,9 +419,8 @@ __device__ __forceinline__ void face_inviscid(const ChemParams &C, const T *rec,
   }
   const T alpha = T(3.0 / 16.0);
   const T k1 = k[0], k2 = k[1], k3 = k[2];
-  const T kk = k1 * k1 + k2 * k2 + k3 * k3;
-  const T igk = frsqrt(kk);
-  const T gk = kk * igk;
+  T gk, igk;
+  length_and_reciprocal(k1 * k1 + k2 * k2 + k3 * k3, gk, igk);
   const T ul = (k1 * L[1] + k2 * L[2] + k3 * L[3]) * igk;
   const T ur = (k1 * R[1] + k2 * R[2] + k3 * R[3]) * igk;
   const T rho_l = L[0], rho_r = R[0];
