@@ -1237,12 +1237,15 @@ int autotune(cc_ctx *c) {
         (Launch<T, NS>::faces_tma_smem(ty, 32) != 0 || Launch<T, NS>::faces_tma_smem(ty, 16) != 0))
       tys.push_back(ty);
   if (tys.empty()) return fail(CC_ERR_ARG, "the face tile height does not fit in shared memory in this precision");
+  // update kernel forms; FP64 spills in the TMA one (stage_update.cuh), which is
+  // not timed there: it made a small FP64 context's set-up longer for nothing
   std::vector<int> forms{0};
   if (c->precision != CC_FP64) forms.push_back(1);
-  if (c->d_qmaps) forms.push_back(2);
+  if (c->d_qmaps && c->precision != CC_FP64) forms.push_back(2);
   if (const char *oe = std::getenv("CC_UPDATE_OCC")) {  // pins it (profiling runs, whose timings are distorted)
     const int form = std::atoi(oe);
-    forms.assign(1, std::count(forms.begin(), forms.end(), form) ? form : 0);
+    const bool runs = form == 2 ? c->d_qmaps != nullptr : form == 1 && c->precision != CC_FP64;
+    forms.assign(1, runs ? form : 0);
   }
   // tile widths of the TMA face kernels: 32, and 16 (with heights 8 and 16)
   // for variants 3-4, whose narrower tiles waste fewer lanes on blocks whose
@@ -1270,18 +1273,21 @@ int autotune(cc_ctx *c) {
     ms = t / n;
     return 0;
   };
-  // the better of two batches after an untimed launch; before the first
-  // candidate the GPU is kept busy for 10 ms (an idle GPU's first launches are
-  // slow, which made the early candidates lose now and then: 128^3 steps of
-  // 2.55 or 2.9 ms)
+  // the better of two batches after an untimed launch, the second only for a
+  // candidate near the best so far (losers by more than a quarter stay losers);
+  // the first candidate is launched a few times before, against slow first
+  // launches.  An early candidate that lost by chance once made a 128^3 step
+  // 2.9 ms instead of 2.55; launches of a fresh context are steady from the
+  // second on, and 10 ms of them took a third of a shock tube's set-up.
   bool warm = false;
-  auto timed = [&](auto &&launch, double &ms) -> int {
-    double t = 0, busy = 0;
-    for (int n = 0; !warm && busy < 10.0 && n < 2000; ++n, busy += t)
+  auto timed = [&](auto &&launch, double best, double &ms) -> int {
+    double t = 0;
+    for (int n = 0; !warm && n < 8; ++n)
       if (int r = batch(launch, 1, t)) return r;
     warm = true;
     if (int r = launch()) return r;
     if (int r = batch(launch, 2, ms)) return r;
+    if (ms > 1.25 * best) return 0;
     if (int r = batch(launch, 2, t)) return r;
     ms = std::min(ms, t);
     return 0;
@@ -1317,7 +1323,8 @@ int autotune(cc_ctx *c) {
           c->upd_form = form;
           if (int r = set_update_tiles(kz, ux)) return r;
           double ms = 0;
-          if (int r = timed([&] { return launch_update<T, NS>(c, u, c->d_utiles, (int)c->hutiles.size()); }, ms)) return r;
+          if (int r = timed([&] { return launch_update<T, NS>(c, u, c->d_utiles, (int)c->hutiles.size()); }, upd_ms, ms))
+            return r;
           if (verbose)
             std::fprintf(stderr, "cc autotune: update form %d tile %dx%dx%d %.4f ms\n", form, ux, 256 / ux, kz, ms);
           if (ms < upd_ms) upd_ms = ms, upd_kz = kz, upd_tx = ux, upd_form = form;
@@ -1347,12 +1354,12 @@ int autotune(cc_ctx *c) {
           auto launch = [&] {
             return is_split ? launch_faces<T, NS>(c, a, pc, variant, nt, n_edge, c->d_ftiles, n_ft) : launch_whole(variant);
           };
-          if (int r = timed(launch, ms)) return r;
+          Best &best = is_split ? split : whole;
+          if (int r = timed(launch, is_split ? best.ms - upd_ms : best.ms, ms)) return r;
           if (is_split) ms += upd_ms;
           if (verbose)
             std::fprintf(stderr, "cc autotune: %s tile %dx%dx%d tiles=%d %.4f ms\n", kVariantName[variant],
                          variant >= 3 ? tx : kTX, variant >= 3 ? ty : kTY, kz, variant >= 3 ? n_ft : nt, ms);
-          Best &best = is_split ? split : whole;
           if (ms < best.ms) best = Best{ms, variant, kz, ty, tx};
         }
       }
@@ -1360,7 +1367,7 @@ int autotune(cc_ctx *c) {
   }
   if (split.ms < 1e300) {
     if (int r = set_tiles(split.kz, split.ty, split.tx)) return r;
-    if (int r = timed([&] { return launch_whole(split.variant); }, split.ms)) return r;
+    if (int r = timed([&] { return launch_whole(split.variant); }, 1e300, split.ms)) return r;
   }
   const Best best = split.ms < whole.ms ? split : whole;
   cudaEventDestroy(e0);
