@@ -102,7 +102,7 @@ CCB_HD constexpr int face_stride(int nv, int elem) {
 // First value of direction d in the face arena of N points.  Offsets within a
 // direction stay below n_var N and are formed in 32 bits (arena_fits); three
 // directions together may not.
-CCB_HD constexpr int64_t face_base(int d, int nv, int elem, int64_t N) { return (int64_t)d * face_stride(nv, elem) * N; }
+CCB_HD constexpr int64_t face_base(int d, int nv, int elem, int N) { return (int64_t)(d * face_stride(nv, elem)) * N; }
 
 // Whether 32-bit offsets reach every field of an arena of N points: at most
 // 6 + kMaxSpec fields per array (per direction of the face arena).

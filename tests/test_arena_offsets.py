@@ -31,7 +31,7 @@ int main() {
       const int64_t inner = elem == 8 ? (int64_t)(nv - 1) * N : (int64_t)4 * ((nv - 1) / 4) * N;
       if (inner >= lim) return 3;
       for (int d = 0; d < 3; ++d) {
-        const int64_t at = face_base(d, nv, elem, N);
+        const int64_t at = face_base(d, nv, elem, (int)N);
         if (at != d * (int64_t)stride * N) return 4;
         const int width = elem == 8 ? 1 : (nv - (nv - 1) / 4 * 4 > 2 ? 4 : 2);
         if (at + inner + (int64_t)width * N > total) return 5;  // the last group of the last point
