@@ -190,7 +190,8 @@ struct GridBarrier {
 constexpr int kHaloMaxLevels = 32;
 constexpr int kHaloFewLevels = 8;        // always in one launch
 constexpr int64_t kHaloWideNodes = 1 << 18;  // more levels than that: while no level has more nodes
-constexpr int kHaloTailNodes = 128;  // a tail level (run by one CTA, one node a thread) has at most this many nodes
+constexpr int kHaloThreads = 128;              // CTA size of the node level kernels
+constexpr int kHaloTailNodes = kHaloThreads;   // a tail level (run by one CTA, a node a thread) has at most this many nodes
 struct HaloLevels {
   int64_t begin[kHaloMaxLevels + 1];
   int n;

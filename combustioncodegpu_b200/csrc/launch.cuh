@@ -354,7 +354,7 @@ cudaError_t Launch<T, NS>::halo_copies(const HaloArgs<T> &a, const ChemParams &C
 template <typename T, int NS>
 cudaError_t Launch<T, NS>::halo_levels(const HaloArgs<T> &a, const ChemParams &C, const HaloLevels &lv,
                                        GridBarrier *bar, unsigned *status, cudaStream_t s) {
-  const int tpb = 128;
+  const int tpb = kHaloThreads;
   static int capacity = 0;  // CTAs that fit on the device at once
   if (capacity == 0) {
     int dev = 0, n_sm = 0, per_sm = 0;

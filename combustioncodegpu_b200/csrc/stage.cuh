@@ -1046,7 +1046,7 @@ __device__ __forceinline__ bool grid_sync_bounded(GridBarrier *bar, long long ma
 // the last eight hold less than a CTA's worth of nodes each and cost a launch
 // or a grid barrier more than their work.
 template <typename T, int NS>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(kHaloThreads)
     k_halo_levels(const HaloArgs<T> a, const __grid_constant__ ChemParams C, const HaloLevels lv, GridBarrier *bar,
                   unsigned *status) {
   const int64_t tid = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -1060,7 +1060,7 @@ __global__ void __launch_bounds__(128)
       return;
     }
     if (tail && blockIdx.x != 0) return;
-    for (int64_t e = lv.begin[l] + (tail ? threadIdx.x : tid); e < lv.begin[l + 1]; e += stride)
+    for (int64_t e = lv.begin[l] + (tail ? threadIdx.x : tid); e < lv.begin[l + 1]; e += tail ? blockDim.x : stride)
       halo_node<T, NS>(a, C, e);
   }
 }
