@@ -31,6 +31,7 @@ MAX_SPECIES = 16
 CC_FP64, CC_MIXED, CC_FP32 = 0, 1, 2
 CC_RK3, CC_STEADY_EULER, CC_STEADY_LUSGS = 0, 1, 2
 PRECISIONS = {"fp64": CC_FP64, "mixed": CC_MIXED, "fp32": CC_FP32}
+UPDATE_FORMS = ("plain", "plain-4", "tma")  # update kernel forms, cc_update_tuning order
 VARIANTS = ("l1", "tma", "split", "split-tma", "split-tma-p", "dq-tma")  # stage-kernel variants, cc_tuning order
 SCHEMES = {"rk3": CC_RK3, "steady": CC_STEADY_EULER, "lusgs": CC_STEADY_LUSGS}
 
@@ -111,6 +112,8 @@ EXPORTS = {
                    ctypes.POINTER(ctypes.c_int)], ctypes.c_int),
     "cc_set_tuning": ([ctypes.c_void_p, ctypes.c_int, ctypes.c_int, ctypes.c_int], ctypes.c_int),
     "cc_set_launch_mode": ([ctypes.c_void_p, ctypes.c_int], ctypes.c_int),
+    "cc_update_tuning": ([ctypes.c_void_p, ctypes.POINTER(ctypes.c_int), ctypes.POINTER(ctypes.c_int)], ctypes.c_int),
+    "cc_set_update_tuning": ([ctypes.c_void_p, ctypes.c_int, ctypes.c_int], ctypes.c_int),
     "cc_set_tile_width": ([ctypes.c_void_p, ctypes.c_int], ctypes.c_int),
     "cc_set_closure": ([ctypes.c_void_p, ctypes.c_void_p], ctypes.c_int),
     "cc_use_closure": ([ctypes.c_void_p, ctypes.c_int], ctypes.c_int),
@@ -472,6 +475,20 @@ class Driver:
         v = (-1 if variant == "auto" else VARIANTS.index(variant)) if isinstance(variant, str) else int(variant)
         _check(self.lib.cc_set_tile_width(self.ctx, int(tile_i)))
         _check(self.lib.cc_set_tuning(self.ctx, v, int(kz), int(tile_j)))
+
+    def update_tuning(self):
+        """Update kernel of the split variants: form ("plain", "plain-4" at
+        four CTAs per SM, "tma"; None while a fused variant is in use) and its
+        tile (i, j, k) in points."""
+        form, tile = ctypes.c_int(), (ctypes.c_int * 3)()
+        _check(self.lib.cc_update_tuning(self.ctx, ctypes.byref(form), tile))
+        return {"form": None if form.value < 0 else UPDATE_FORMS[form.value], "tile": tuple(tile)}
+
+    def set_update_tuning(self, form="auto", tile_i=0):
+        """Pin the update kernel's form ("auto" or one of UPDATE_FORMS) and
+        tile width (32, 16; 0 = autotune) from the next tuning on."""
+        f = -1 if form == "auto" else UPDATE_FORMS.index(form)
+        _check(self.lib.cc_set_update_tuning(self.ctx, f, int(tile_i)))
 
     def set_launch_mode(self, mode="batched"):
         """"batched": one launch per stage kernel over all blocks;

@@ -109,6 +109,8 @@ struct cc_ctx {
   int upd_form = 0;               // autotuned: 0 = k_update, 1 = the same sized for 4 CTAs per SM instead of 3 (FP32),
                                   // 2 = k_update_tma
   int upd_kz = 1;                 // k-planes per update tile
+  int force_form = -1;            // cc_set_update_tuning: update kernel form, -1 = autotune
+  int force_ux = 0;               // cc_set_update_tuning: update tile width, 0 = autotune
   int force_ty = 0;               // cc_set_tuning: face tile height, 0 = autotune
   std::vector<Tile> hutiles;      // variants 2-5: tiles of the update kernel (upd_tx x 256/upd_tx x kz)
   std::vector<int> ut_begin;      // per block: first update tile, + end
@@ -1187,7 +1189,8 @@ int lusgs_alloc(cc_ctx *c) {
 template <typename T, int NS>
 int autotune(cc_ctx *c) {
   const char *env = std::getenv("CC_AUTOTUNE");
-  if (env && env[0] == '0' && c->force_variant < 0 && c->force_kz <= 0) return 0;
+  if (env && env[0] == '0' && c->force_variant < 0 && c->force_kz <= 0 && c->force_form < 0 && c->force_ux <= 0)
+    return 0;
   const char *venv = std::getenv("CC_AUTOTUNE_VERBOSE");  // print every candidate's time to stderr
   const bool verbose = venv && venv[0] == '1';
   StageArgs<T> a{};
@@ -1242,11 +1245,17 @@ int autotune(cc_ctx *c) {
   std::vector<int> forms{0};
   if (c->precision != CC_FP64) forms.push_back(1);
   if (c->d_qmaps && c->precision != CC_FP64) forms.push_back(2);
-  if (const char *oe = std::getenv("CC_UPDATE_OCC")) {  // pins it (profiling runs, whose timings are distorted)
+  auto runs = [&](int form) { return form == 0 || (form == 1 ? c->precision != CC_FP64 : c->d_qmaps != nullptr); };
+  if (c->force_form >= 0 && !runs(c->force_form))
+    return fail(CC_ERR_ARG, "the update kernel form needs the FP32 bulk precision (1) or tensor maps (2) "
+                            "(cc_set_update_tuning)");
+  if (c->force_form >= 0)
+    forms.assign(1, c->force_form);
+  else if (const char *oe = std::getenv("CC_UPDATE_OCC")) {  // the same for profiling runs; 0 where a form does not run
     const int form = std::atoi(oe);
-    const bool runs = form == 2 ? c->d_qmaps != nullptr : form == 1 && c->precision != CC_FP64;
-    forms.assign(1, runs ? form : 0);
+    forms.assign(1, form >= 0 && form <= 2 && runs(form) ? form : 0);
   }
+  const std::vector<int> uxs = c->force_ux > 0 ? std::vector<int>{c->force_ux} : std::vector<int>{32, 16};
   // tile widths of the TMA face kernels: 32, and 16 (with heights 8 and 16)
   // for variants 3-4, whose narrower tiles waste fewer lanes on blocks whose
   // extent is not a multiple of 32
@@ -1318,7 +1327,7 @@ int autotune(cc_ctx *c) {
     u.faces = (T *)c->faces;
     u.a = 0.75, u.b = 0.25;
     for (int form : forms)
-      for (int ux : {32, 16})
+      for (int ux : uxs)
         for (int kz : ukzs) {
           c->upd_form = form;
           if (int r = set_update_tiles(kz, ux)) return r;
@@ -2001,6 +2010,23 @@ int cc_tuning(cc_ctx *c, int *variant, int *kz, double *stage_ms, int tile[3]) {
     tile[1] = c->variant >= 3 ? c->face_ty : kTY;
     tile[2] = c->kz;
   }
+  return 0;
+}
+
+int cc_update_tuning(cc_ctx *c, int *form, int tile[3]) {
+  if (int r = check_ctx(c)) return r;
+  if (form) *form = c->variant >= 2 ? c->upd_form : -1;
+  if (tile) tile[0] = c->upd_tx, tile[1] = 256 / c->upd_tx, tile[2] = c->upd_kz;
+  return 0;
+}
+
+int cc_set_update_tuning(cc_ctx *c, int form, int tile_i) {
+  if (int r = check_ctx(c)) return r;
+  if (form < -1 || form > 2)
+    return fail(CC_ERR_ARG, "form must be -1 (autotune), 0 (plain), 1 (plain, 4 CTAs per SM) or 2 (state by TMA)");
+  if (tile_i != 0 && tile_i != 16 && tile_i != 32) return fail(CC_ERR_ARG, "tile_i must be 0 (autotune), 16 or 32");
+  c->force_form = form;
+  c->force_ux = tile_i;
   return 0;
 }
 

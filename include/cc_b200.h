@@ -223,8 +223,9 @@ int cc_tuning(cc_ctx *ctx, int *variant, int *kz, double *stage_ms, int tile[3])
  * instead of autotuning it: variant -1 = autotune, 0 = fused with L1 stencil
  * reads, 1 = fused with TMA-staged planes, 2 = split faces / update, 3 =
  * split with TMA-staged face planes, 4 = as 3 on persistent CTAs, 5 = faces
- * differenced in the tile (TMA variants: 0 or 9 species; 1 and 5: FP32 bulk
- * precision); kz = k-planes per tile, 0 = autotune; tile_j = points along j
+ * differenced in the tile (TMA variants can be pinned with 0 or 9 species, 1
+ * and 5 in the FP32 bulk precision only; the autotuner also takes 3 with other
+ * counts); kz = k-planes per tile, 0 = autotune; tile_j = points along j
  * of the TMA face kernel's tile in variants 3-5 (4, 8 or 16, 16 in the FP32
  * bulk precision only; 0 = autotune; the other kernels' tiles are 32 x 8).
  * Before cc_init it applies to the first cc_init; after it, the new
@@ -236,6 +237,17 @@ int cc_set_tuning(cc_ctx *ctx, int variant, int kz, int tile_j);
  * autotune (default).  Applies from the next tuning: cc_init or
  * cc_set_tuning. */
 int cc_set_tile_width(cc_ctx *ctx, int tile_i);
+/* The update kernel of the split variants (2-5), which is timed apart from the
+ * face kernel: form 0 = conserved states by plain loads, 1 = the same at four
+ * CTAs per SM (FP32 bulk precision), 2 = conserved states staged by TMA; tiles
+ * of 32 x 8 or 16 x 16 points.  cc_update_tuning reports the form (-1 while a
+ * fused variant is in use) and its tile {i, j, k}; either may be null.
+ * cc_set_update_tuning pins the form (-1 = autotune) and the tile width (0 =
+ * autotune) from the next tuning on: cc_init or cc_set_tuning, which fail with
+ * CC_ERR_ARG when the form does not run in the context.  Every form gives the
+ * same states bit for bit. */
+int cc_update_tuning(cc_ctx *ctx, int *form, int tile[3]);
+int cc_set_update_tuning(cc_ctx *ctx, int form, int tile_i);
 /* Launch granularity of the stage kernels: 0 (default) = one launch per
  * kernel over the tiles of every block; 1 = one launch per block per kernel,
  * the reference's granularity (Driver.cu:144-177 launches per block), kept for
