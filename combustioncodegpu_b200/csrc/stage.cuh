@@ -336,12 +336,8 @@ __device__ __forceinline__ double stage_value(const ChemParams &C, const StageAr
 template <typename T>
 __device__ __forceinline__ double conserved_update(const ChemParams &C, const StageArgs<T> &a, int p, int N, int l,
                                                    double dql, double dtj, bool three_d) {
-  if (a.gcl && l >= 1 && l <= 3) dql -= C.p_ref * a.gcl[(l - 1) * N + p];
-  double qs = a.Qin[l * N + p] + dql * dtj;
-  if (l == 3 && !three_d) qs = 0;
-  double q = (a.a != 0.0) ? a.a * a.Qn[l * N + p] + a.b * qs : qs;
-  if (a.q32) q = (double)(float)q;
-  return q;
+  const double gcl = a.gcl && l >= 1 && l <= 3 ? a.gcl[(l - 1) * N + p] : 0.0;
+  return stage_value<T>(C, a, l, dql, gcl, dtj, three_d, a.Qin[l * N + p], a.a != 0.0 ? a.Qn[l * N + p] : 0.0);
 }
 
 // Stores the new conserved state q of point p, recovers its primitives (FP64
