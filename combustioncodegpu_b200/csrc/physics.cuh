@@ -38,17 +38,38 @@ struct SpecCount {
 
 // Division, reciprocal, square root and x^-0.145 of the bulk precision: IEEE
 // in FP64 (the plain path), hardware approximations in FP32 (the mixed path;
-// relative error of a few ulp, far below the path's 1e-5 error budget).  The
-// FP32 forms take denormal operands: a density of 1e-40 is far from any flow,
-// but flushed to zero it divides to infinity.  Flushing forms (.ftz), which
-// save the scaling of operands, were faster by 1.3 % of a 128^3 mixed step
-// (2.618 against 2.656 ms).
+// relative error of a few ulp, far below the path's 1e-5 error budget).
+// These take denormal operands: a density of 1e-40 is far from any flow, but
+// flushed to zero it divides to infinity.
 __device__ __forceinline__ double fdiv(double a, double b) { return a / b; }
 __device__ __forceinline__ float fdiv(float a, float b) { return __fdividef(a, b); }
 __device__ __forceinline__ double frcp(double a) { return 1.0 / a; }
 __device__ __forceinline__ float frcp(float a) { return __fdividef(1.0f, a); }
 __device__ __forceinline__ double fsqrt(double a) { return sqrt(a); }
 __device__ __forceinline__ float fsqrt(float a) { return a * rsqrtf(a); }
+
+// The same where the operand taken by the hardware is a normal number whatever
+// the state's density and pressure: sums over mole fractions that add up to
+// one, specific heats, a temperature and what is formed of it and the species'
+// constants (normal down to 1e-30 K).  Numerators may be denormal.  These
+// flush denormal operands (.ftz), which saves the scaling of every operand:
+// the update of 128^3 mixed takes 0.314 ms a stage with them and 0.318 with the
+// others, the halo program of 12 blocks 0.307 and 0.320, the 128^3 step 2.637 and
+// 2.655.
+__device__ __forceinline__ double rcp_normal(double a) { return 1.0 / a; }
+__device__ __forceinline__ float rcp_normal(float a) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a));
+  return r;
+}
+__device__ __forceinline__ double div_normal(double a, double b) { return a / b; }
+__device__ __forceinline__ float div_normal(float a, float b) { return a * rcp_normal(b); }
+__device__ __forceinline__ double sqrt_normal(double a) { return sqrt(a); }
+__device__ __forceinline__ float sqrt_normal(float a) {
+  float r;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a));
+  return a * r;
+}
 
 // Length of the face vector, from its square, and the reciprocal of that
 // length.  The mass flux takes the product of both, so what counts is that
@@ -192,7 +213,10 @@ __device__ __forceinline__ double pow_m0145<double>(double x) {
 }
 template <>
 __device__ __forceinline__ float pow_m0145<float>(float x) {
-  return __powf(x, -0.145f);
+  float l, r;  // x: reduced temperature
+  asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(l) : "f"(x));
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(-0.145f * l));
+  return r;
 }
 
 // Wilke mixture viscosity, modified-Wilke conductivity and constant-Schmidt
@@ -204,17 +228,17 @@ __device__ __forceinline__ void transport(const ChemParams &C, T temp, const T *
   constexpr int A = SpecCount<NS>::kArr;
   const int ns = SpecCount<NS>::n(C);
   T X[A], vis[A], svis[A], isvis[A];
-  const T sqt = fsqrt(temp);
+  const T sqt = sqrt_normal(temp);
 #pragma unroll
   for (int l = 0; l < A; ++l) {
     if (l < ns) {
       X[l] = Y[l] * mw_total * S.inv_mw[l];
       const T t_dl = temp * S.lj_inv[l];
       const T tp = t_dl + T(0.5);
-      const T omega = T(1.147) * pow_m0145<T>(t_dl) + frcp(tp * tp);
-      vis[l] = fdiv(S.vis_coeff[l] * sqt, omega);
-      svis[l] = fsqrt(vis[l]);
-      isvis[l] = frcp(svis[l]);
+      const T omega = T(1.147) * pow_m0145<T>(t_dl) + rcp_normal(tp * tp);
+      vis[l] = div_normal(S.vis_coeff[l] * sqt, omega);
+      svis[l] = sqrt_normal(vis[l]);
+      isvis[l] = rcp_normal(svis[l]);
     }
   }
   T viscosity = 0, conductivity = 0;
@@ -236,8 +260,8 @@ __device__ __forceinline__ void transport(const ChemParams &C, T temp, const T *
         }
       }
       const T lam_m = vis[m] * (cp[m] + S.lam_shift[m]);
-      viscosity += fdiv(vis[m] * X[m], vt);
-      conductivity += fdiv(lam_m * X[m], T(1.065) * vt - T(0.065) * X[m]);
+      viscosity += div_normal(vis[m] * X[m], vt);
+      conductivity += div_normal(lam_m * X[m], T(1.065) * vt - T(0.065) * X[m]);
     }
   }
   mu_out = viscosity;
@@ -247,7 +271,7 @@ __device__ __forceinline__ void transport(const ChemParams &C, T temp, const T *
   for (int l = 0; l < A; ++l) {
     if (l < ns) {
       const T d = X[l] - T(1);
-      rhod[l] = (fabs(d) < T(1e-3)) ? viscosity * inv_sc : fdiv((T(1) - Y[l]) * viscosity, (T(1) - X[l]) * T(C.Sc));
+      rhod[l] = (fabs(d) < T(1e-3)) ? viscosity * inv_sc : div_normal((T(1) - Y[l]) * viscosity, (T(1) - X[l]) * T(C.Sc));
     }
   }
 }
@@ -276,9 +300,9 @@ __device__ __forceinline__ void point_props(const ChemParams &C, const T *rec, T
   for (int l = 0; l < A; ++l)
     if (l < ns) mwi += Y[l] * S.inv_mw[l], cp_mix += Y[l] * cp[l];
   const T gas = T(kRu) * mwi;
-  gamma = fdiv(cp_mix, cp_mix - gas);
-  c = fsqrt(gamma * gas * temp);
-  transport<T, NS>(C, temp, Y, frcp(mwi), cp, mu, lam, rhod);
+  gamma = div_normal(cp_mix, cp_mix - gas);
+  c = sqrt_normal(gamma * gas * temp);
+  transport<T, NS>(C, temp, Y, rcp_normal(mwi), cp, mu, lam, rhod);
 }
 
 // Temperature from internal energy by Newton iteration (tolerance 1e-3 on

@@ -1,4 +1,4 @@
-"""Density in the FP32 denormal range (2e-41 kg/m3; times the gas constant
+"""Small operands of the FP32 approximations.  Density in the FP32 denormal range (2e-41 kg/m3; times the gas constant
 still below 1.2e-38): the mixed path's FP32 divisions take denormal operands
 instead of flushing them to zero, so a uniform stream stays as it is, as in
 FP64.  Tolerance 5e-4: a few of the relative steps in which FP32 resolves such
@@ -24,6 +24,33 @@ def _uniform(kind, rho=2e-41):
     bv[:] = np.array([rho, 30.0, -20.0, 10.0, rho * gas * 900.0, 900.0])[:, None]
     blk["bv"] = bv
     return case
+
+
+@pytest.mark.parametrize("temperature", [1e-3, 1.0, 40.0, 900.0, 2e4])
+@pytest.mark.parametrize("trace", [1e-3, 1e-30, 1e-41])
+def test_transport_of_traces_and_extreme_temperatures(temperature, trace):
+    """The transport's FP32 approximations flush denormal operands; none is
+    denormal over temperatures beyond any flow's and down to denormal mass
+    fractions: as in FP64 within 1e-5, the path's error budget."""
+    props = []
+    for precision in ("fp64", "mixed"):
+        case = _uniform("mixture", rho=1.0)
+        blk = case["blocks"][0]
+        y = np.full(9, trace)
+        y[8] = 1.0 - y[:8].sum()
+        blk["yk"][:] = y[:, None]
+        gas = cases.R_U * (y / np.asarray(case["params"]["species"]["mw"])).sum()
+        blk["bv"][5] = temperature
+        blk["bv"][4] = gas * temperature
+        d = cc.Driver.from_case(case, precision)
+        d.set_tuning("split", 2)
+        d.initialize_computation()
+        d.simulate(1)
+        assert d.status() == 0
+        props.append(d.field[0].get_props())
+        d.close()
+    for want, got in zip(*props):
+        np.testing.assert_allclose(got, want, rtol=1e-5)
 
 
 @pytest.mark.parametrize("kind", ["air", "mixture"])
