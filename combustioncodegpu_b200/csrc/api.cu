@@ -1326,6 +1326,10 @@ int autotune(cc_ctx *c) {
     StageArgs<T> u = a;
     u.faces = (T *)c->faces;
     u.a = 0.75, u.b = 0.25;
+    // the faces of the current state: the arena may hold the dq variant's
+    // residual, of which every form makes states that the Newton iterates on
+    // (128^3: 2.0 to 3.9 ms, and the wrong form chosen)
+    if (int r = launch_faces<T, NS>(c, a, pc, 2, (int)c->htiles.size(), (int)c->hedges.size(), nullptr, 0)) return r;
     for (int form : forms)
       for (int ux : uxs)
         for (int kz : ukzs) {
