@@ -964,25 +964,29 @@ bool variant_tried(const cc_ctx *c, int v) {
   return variant_ok(c, v) || (v == 3 && c->tma_ok);
 }
 
-// One stage's kernels of the given variant over the current tile list:
-// one launch per kernel over all blocks, or (per_block) one per block.
-template <typename T, int NS>
-int launch_stage_range(cc_ctx *c, StageArgs<T> a, int pc, int variant, int nt, int n_edge, const Tile *face_tiles,
-                       int n_ft, const Tile *upd_tiles, int n_ut);
+// A range of the current tile lists, launched together: every block's, or
+// (per_block) one block's.
+struct TileRange {
+  int nt, n_edge;  // of StageArgs::tiles and edge_tiles
+  const Tile *face_tiles;
+  int n_ft;
+  const Tile *upd_tiles;
+  int n_ut;
+};
 
-template <typename T, int NS>
-int launch_stage(cc_ctx *c, StageArgs<T> a, int pc, int variant, int nt) {
+// f(a, range) for every range of the context's launch mode.
+template <typename T, typename F>
+int each_range(cc_ctx *c, StageArgs<T> a, F &&f) {
   if (!c->per_block || c->tile_begin.size() != c->blocks.size() + 1)
-    return launch_stage_range<T, NS>(c, a, pc, variant, nt, (int)c->hedges.size(), c->d_ftiles,
-                                     (int)c->hftiles.size(), c->d_utiles, (int)c->hutiles.size());
+    return f(a, TileRange{(int)c->htiles.size(), (int)c->hedges.size(), c->d_ftiles, (int)c->hftiles.size(),
+                          c->d_utiles, (int)c->hutiles.size()});
   const Tile *tiles = a.tiles;
   for (size_t b = 0; b < c->blocks.size(); ++b) {
     a.tiles = tiles + c->tile_begin[b];
     a.edge_tiles = c->d_edges + c->edge_begin[b];
-    if (int r = launch_stage_range<T, NS>(c, a, pc, variant, c->tile_begin[b + 1] - c->tile_begin[b],
-                                          c->edge_begin[b + 1] - c->edge_begin[b], c->d_ftiles + c->ft_begin[b],
-                                          c->ft_begin[b + 1] - c->ft_begin[b], c->d_utiles + c->ut_begin[b],
-                                          c->ut_begin[b + 1] - c->ut_begin[b]))
+    if (int r = f(a, TileRange{c->tile_begin[b + 1] - c->tile_begin[b], c->edge_begin[b + 1] - c->edge_begin[b],
+                               c->d_ftiles + c->ft_begin[b], c->ft_begin[b + 1] - c->ft_begin[b],
+                               c->d_utiles + c->ut_begin[b], c->ut_begin[b + 1] - c->ut_begin[b]}))
       return r;
   }
   return 0;
@@ -1006,49 +1010,56 @@ int launch_update(cc_ctx *c, StageArgs<T> a, const Tile *upd_tiles, int n_ut) {
 // The face kernels of the split variants (2-4): every face flux of the stage
 // into the face arena.
 template <typename T, int NS>
-int launch_faces(cc_ctx *c, StageArgs<T> a, int pc, int variant, int nt, int n_edge, const Tile *face_tiles,
-                 int n_ft) {
+int launch_faces(cc_ctx *c, StageArgs<T> a, int pc, int variant, const TileRange &g) {
   a.faces = (T *)c->faces;
   if (!a.edge_tiles) a.edge_tiles = c->d_edges;
   if (variant == 2) {
-    CK((Launch<T, NS>::faces(a, c->chem, nt, n_edge, c->stream)));
+    CK((Launch<T, NS>::faces(a, c->chem, g.nt, g.n_edge, c->stream)));
     return 0;
   }
   // regular tiles from TMA-staged planes (persistent CTAs for 4), edge tiles through L1
   const CUtensorMap *maps = c->d_tmaps + ((size_t)tma_shape(c->face_ty, c->face_tx) * 2 + pc) * c->blocks.size();
   if (variant == 3)
-    CK((Launch<T, NS>::faces_tma(a, face_tiles, c->face_ty, c->face_tx, maps, c->chem, n_ft, c->stream)));
+    CK((Launch<T, NS>::faces_tma(a, g.face_tiles, c->face_ty, c->face_tx, maps, c->chem, g.n_ft, c->stream)));
   else
-    CK((Launch<T, NS>::faces_tma_persistent(a, face_tiles, c->face_ty, c->face_tx, maps, c->chem, n_ft, c->d_ticket,
-                                            c->stream)));
-  CK((Launch<T, NS>::faces(a, c->chem, 0, n_edge, c->stream)));
+    CK((Launch<T, NS>::faces_tma_persistent(a, g.face_tiles, c->face_ty, c->face_tx, maps, c->chem, g.n_ft,
+                                            c->d_ticket, c->stream)));
+  CK((Launch<T, NS>::faces(a, c->chem, 0, g.n_edge, c->stream)));
   return 0;
 }
 
 template <typename T, int NS>
-int launch_stage_range(cc_ctx *c, StageArgs<T> a, int pc, int variant, int nt, int n_edge, const Tile *face_tiles,
-                       int n_ft, const Tile *upd_tiles, int n_ut) {
+int launch_stage_range(cc_ctx *c, StageArgs<T> a, int pc, int variant, const TileRange &g) {
   if ((variant == 1 || variant == 3 || variant == 4 || variant == 5) && !c->d_tmaps)
     return fail(CC_ERR_STATE, "TMA variant without tensor maps");
   if (variant == 0) {
-    CK((Launch<T, NS>::stage(a, c->chem, nt, c->stream)));
+    CK((Launch<T, NS>::stage(a, c->chem, g.nt, c->stream)));
     return 0;
   }
   if (variant == 1) {
-    CK((Launch<T, NS>::stage_tma(a, c->d_tmaps + (size_t)pc * c->blocks.size(), c->chem, nt, c->stream)));
+    CK((Launch<T, NS>::stage_tma(a, c->d_tmaps + (size_t)pc * c->blocks.size(), c->chem, g.nt, c->stream)));
     return 0;
   }
   a.faces = (T *)c->faces;
   if (variant == 5) {  // faces differenced in the tile (dq), then the update
     a.dq_direct = 1;
     const size_t nb = c->blocks.size();
-    CK((Launch<T, NS>::faces_dq(a, face_tiles, c->d_tmaps + ((size_t)tma_shape(c->face_ty) * 2 + pc) * nb, c->chem,
-                                n_ft, c->face_ty, c->stream)));
-  } else if (int r = launch_faces<T, NS>(c, a, pc, variant, nt, n_edge, face_tiles, n_ft)) {
+    CK((Launch<T, NS>::faces_dq(a, g.face_tiles, c->d_tmaps + ((size_t)tma_shape(c->face_ty) * 2 + pc) * nb, c->chem,
+                                g.n_ft, c->face_ty, c->stream)));
+  } else if (int r = launch_faces<T, NS>(c, a, pc, variant, g)) {
     return r;
   }
   if (int r = prof_event(c, c->ev_mid, c->ev_next_mid)) return r;
-  return launch_update<T, NS>(c, a, upd_tiles, n_ut);
+  return launch_update<T, NS>(c, a, g.upd_tiles, g.n_ut);
+}
+
+// One stage's kernels of the given variant: one launch per kernel over all
+// blocks, or (per_block) one per block.
+template <typename T, int NS>
+int launch_stage(cc_ctx *c, const StageArgs<T> &a, int pc, int variant) {
+  return each_range<T>(c, a, [&](const StageArgs<T> &ra, const TileRange &g) {
+    return launch_stage_range<T, NS>(c, ra, pc, variant, g);
+  });
 }
 
 // The closure transport of the new state (when on), the end of the stage's
@@ -1068,9 +1079,8 @@ int after_stage(cc_ctx *c, const StageArgs<T> &a, int pn, int pc, double *qout, 
 template <typename T, int NS>
 int stage_and_halo(cc_ctx *c, const StageArgs<T> &a, int pn, int pc, double *qout, const double *qin,
                    int stage = 0) {
-  const int nt = (int)c->htiles.size();
   if (int r = prof_event(c, c->ev_stage, c->ev_next_stage)) return r;
-  if (int r = launch_stage<T, NS>(c, a, pc, c->variant, nt)) return r;
+  if (int r = launch_stage<T, NS>(c, a, pc, c->variant)) return r;
   return after_stage<T, NS>(c, a, pn, pc, qout, qin, stage);
 }
 
@@ -1184,8 +1194,9 @@ int lusgs_alloc(cc_ctx *c) {
 // fused variants as a whole (kernel x k-chunk); for the split variants the
 // face kernel (variant x tile x k-chunk) and the update kernel (form x tile x
 // k-chunk) each by itself, since neither's choice changes the other's time,
-// and their best as a whole.  The candidates write only the scratch halves of
-// the ping-pong buffers and the face arena, so the state is unchanged.
+// and their best as a whole; all of it in the context's launch mode.  The
+// candidates write only the scratch halves of the ping-pong buffers and the
+// face arena, so the state is unchanged.
 template <typename T, int NS>
 int autotune(cc_ctx *c) {
   const char *env = std::getenv("CC_AUTOTUNE");
@@ -1314,6 +1325,11 @@ int autotune(cc_ctx *c) {
     build_update_tiles(c, kz, ux);
     return upload_update_tiles(c);
   };
+  auto faces = [&](int variant) {
+    return each_range<T>(c, a, [&](const StageArgs<T> &ra, const TileRange &g) {
+      return launch_faces<T, NS>(c, ra, pc, variant, g);
+    });
+  };
   // the update kernel, with the step's-start state read as in two of three RK stages
   double upd_ms = 0;
   int upd_kz = c->kz, upd_tx = 32, upd_form = 0;
@@ -1329,15 +1345,19 @@ int autotune(cc_ctx *c) {
     // the faces of the current state: the arena may hold the dq variant's
     // residual, of which every form makes states that the Newton iterates on
     // (128^3: 2.0 to 3.9 ms, and the wrong form chosen)
-    if (int r = launch_faces<T, NS>(c, a, pc, 2, (int)c->htiles.size(), (int)c->hedges.size(), nullptr, 0)) return r;
+    if (int r = faces(2)) return r;
+    auto update = [&] {
+      return each_range<T>(c, u, [&](const StageArgs<T> &ra, const TileRange &g) {
+        return launch_update<T, NS>(c, ra, g.upd_tiles, g.n_ut);
+      });
+    };
     for (int form : forms)
       for (int ux : uxs)
         for (int kz : ukzs) {
           c->upd_form = form;
           if (int r = set_update_tiles(kz, ux)) return r;
           double ms = 0;
-          if (int r = timed([&] { return launch_update<T, NS>(c, u, c->d_utiles, (int)c->hutiles.size()); }, upd_ms, ms))
-            return r;
+          if (int r = timed(update, upd_ms, ms)) return r;
           if (verbose)
             std::fprintf(stderr, "cc autotune: update form %d tile %dx%dx%d %.4f ms\n", form, ux, 256 / ux, kz, ms);
           if (ms < upd_ms) upd_ms = ms, upd_kz = kz, upd_tx = ux, upd_form = form;
@@ -1352,27 +1372,22 @@ int autotune(cc_ctx *c) {
     double ms = 1e300;
     int variant = 0, kz = 1, ty = 8, tx = 32;
   } split, whole;
-  auto launch_whole = [&](int variant) {
-    return launch_stage_range<T, NS>(c, a, pc, variant, (int)c->htiles.size(), (int)c->hedges.size(), c->d_ftiles,
-                                     (int)c->hftiles.size(), c->d_utiles, (int)c->hutiles.size());
-  };
+  auto launch_whole = [&](int variant) { return launch_stage<T, NS>(c, a, pc, variant); };
   for (int variant : variants) {
     const bool is_split = variant >= 2 && variant <= 4;
     for (int ty : (variant >= 3 ? tys : std::vector<int>{8})) {
       for (int tx : txs_of(variant, ty)) {
         for (int kz : kzs) {
           if (int r = set_tiles(kz, ty, tx)) return r;
-          const int nt = (int)c->htiles.size(), n_edge = (int)c->hedges.size(), n_ft = (int)c->hftiles.size();
           double ms = 0;
-          auto launch = [&] {
-            return is_split ? launch_faces<T, NS>(c, a, pc, variant, nt, n_edge, c->d_ftiles, n_ft) : launch_whole(variant);
-          };
+          auto launch = [&] { return is_split ? faces(variant) : launch_whole(variant); };
           Best &best = is_split ? split : whole;
           if (int r = timed(launch, is_split ? best.ms - upd_ms : best.ms, ms)) return r;
           if (is_split) ms += upd_ms;
           if (verbose)
             std::fprintf(stderr, "cc autotune: %s tile %dx%dx%d tiles=%d %.4f ms\n", kVariantName[variant],
-                         variant >= 3 ? tx : kTX, variant >= 3 ? ty : kTY, kz, variant >= 3 ? n_ft : nt, ms);
+                         variant >= 3 ? tx : kTX, variant >= 3 ? ty : kTY, kz,
+                         (int)(variant >= 3 ? c->hftiles.size() : c->htiles.size()), ms);
           if (ms < best.ms) best = Best{ms, variant, kz, ty, tx};
         }
       }
