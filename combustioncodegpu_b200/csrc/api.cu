@@ -957,8 +957,9 @@ bool variant_ok(const cc_ctx *c, int v) {
 }
 
 // Variants the autotuner tries: those, without the dq one (slower than the
-// best at every size measured: 0.955 against 0.816 ms per mixed 128^3 stage),
-// and with the TMA face planes of the runtime species counts.
+// best at every size measured, mixed, ms per stage: 128^3 0.949 against 0.758,
+// 112^3 0.716 / 0.555, 12 blocks 0.684 / 0.548, channel 0.157 / 0.137, 32^3
+// 0.045 / 0.030), and with the TMA face planes of the runtime species counts.
 bool variant_tried(const cc_ctx *c, int v) {
   if (v == 5) return false;
   return variant_ok(c, v) || (v == 3 && c->tma_ok);

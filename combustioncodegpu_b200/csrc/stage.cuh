@@ -53,7 +53,7 @@ __device__ __forceinline__ double geo_jac(const double *__restrict__ G, int, int
 // that a face is written and read in a quarter of the instructions: 128^3, 9
 // species, faces 0.479 -> 0.440 ms per stage (with the geometry rows).  FP64:
 // one value per group; pairs cost the update more registers in flight than
-// they save instructions (97 x 85 x 71: update 0.249 -> 0.272 ms, faces equal).
+// they save instructions (97 x 85 x 71: update 0.248 -> 0.272 ms, faces equal).
 template <typename T>
 constexpr int kFaceGroup = sizeof(T) == 4 ? 4 : 1;
 template <typename T, int NV>
@@ -91,7 +91,7 @@ __device__ __forceinline__ void store_group(double *__restrict__ Fd, int N, int,
 // minus-side faces at px, py, pz; without a third direction pz = p, whose
 // difference is zero (the arena starts zeroed): a branch around the loads
 // would keep the compiler from batching them over the groups (97 x 85 x 71
-// FP64: update 0.25 against 0.29 ms per stage).
+// FP64: update 0.248 against 0.29 ms per stage).
 template <typename T>
 __device__ __forceinline__ void face_sum(const T *__restrict__ Fx, const T *__restrict__ Fy, const T *__restrict__ Fz,
                                          int N, int nv, int g, int p, int px, int py, int pz,
@@ -314,10 +314,6 @@ __device__ __forceinline__ void gamma_and_c(const ChemParams &C, const T *rec, T
   c = sqrt(gamma * gas * temp);
 }
 
-// RK update of one interior point (TimeAdvanceFunc.cu:255-290 with the
-// Shu-Osher combination), FP64 primitives and Newton, transport properties of
-// the new state (Field.cu:178-210), |V| for the residual and the point's
-// contribution to the next global time step.
 // The conserved variable l of point p after the RK stage, from its residual
 // dql, the geometric term gcl of its direction (l = 1..3) and the states qin
 // and qn (TimeAdvanceFunc.cu:255-265; SSP-RK3 combination; qn counts when
@@ -333,6 +329,7 @@ __device__ __forceinline__ double stage_value(const ChemParams &C, const StageAr
   if (a.q32) q = (double)(float)q;  // full-FP32 study: FP32 conserved state
   return q;
 }
+// The same with the states read here.
 template <typename T>
 __device__ __forceinline__ double conserved_update(const ChemParams &C, const StageArgs<T> &a, int p, int N, int l,
                                                    double dql, double dtj, bool three_d) {
@@ -468,6 +465,10 @@ __device__ __forceinline__ void point_finish(const ChemParams &C, const T *rec, 
   }
 }
 
+// RK update of one interior point (TimeAdvanceFunc.cu:255-290 with the
+// Shu-Osher combination), FP64 primitives and Newton, transport properties of
+// the new state (Field.cu:178-210), |V| for the residual and the point's
+// contribution to the next global time step.
 template <typename T, int NS>
 __device__ __forceinline__ void point_update(const ChemParams &C, const T *rec, const double *rec_d,
                                              const StageArgs<T> &a, int p, int N,

@@ -10,11 +10,13 @@
 // variable) per state, requested for plane k + 1 as soon as the new state of
 // plane k is in registers, so that the copies run beside the Newton, the
 // transport and the stores of plane k and take no registers.  The faces are
-// read while the box is on its way, all before the first is used.  57 KB per
-// CTA at 9 species, two CTAs of 128 registers per SM.  The autotuner times it
-// against k_update: FP32 takes it (128^3: 0.293 against 0.325 ms per stage),
-// FP64, whose faces and states together spill here, does not (97 x 85 x 71:
-// 0.270 against 0.229 ms).
+// read while the box is on its way, all before the first is used.  60 KB per
+// CTA at 9 species (57 of them the boxes), two CTAs of 128 registers per SM.
+// The autotuner times it against k_update: FP32 takes it (128^3: 0.308 to 0.314
+// against 0.346 ms per stage; the channel's steady step, which reads one state
+// and has a time step per point, 0.054 against 0.061).  FP64, whose faces and
+// states together spill here, would not (97 x 85 x 71: 0.286 against 0.248 ms)
+// and is not timed with it.
 //
 // Waits are bounded as in the face kernel: a CTA whose box does not arrive
 // sets kStatusTmaTimeout, waits (bounded) for its copies and leaves.
