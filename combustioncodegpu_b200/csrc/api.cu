@@ -808,10 +808,11 @@ int run_halo(cc_ctx *c, int pn, int pp, double *qn, const double *qp, unsigned l
   // A program of more than kHaloFewLevels levels takes one launch only while no
   // level has more than kHaloWideNodes nodes.  64 blocks (18 levels, 682 k nodes
   // in the widest), per stage: one cooperative launch 1.63 ms, a launch per
-  // level 1.60, both builds measured in turn.  12 blocks (18 levels, 112 k
-  // averaged points): 0.302 ms in one launch; a launch per level took 0.307
-  // before the tail levels shared a CTA.  The line lies between these two
-  // programs; sizes between them were not measured.
+  // level 1.60, both builds measured in turn.  Periodic layouts of 18 levels in
+  // one launch against the kernels that took one per level: 8 blocks of about
+  // 56^3 0.270 against 0.293 ms, 64 of 12^3 0.190 / 0.194, 27 of 29^3 0.281 /
+  // 0.282, 64 of 23^3 0.335 / 0.332.  The line lies above these and below the 64
+  // blocks; across it the two forms differ by 2 %.
   int64_t widest = 0;
   for (int l = 0; l < n_levels; ++l) widest = std::max(widest, lb[l + 1] - lb[l]);
   const bool one_launch = n_levels <= kHaloFewLevels || (n_levels <= kHaloMaxLevels && widest <= kHaloWideNodes);
